@@ -85,6 +85,12 @@ int32_t pdlpgpu_gemm_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, co
 int32_t pdlpgpu_encode_features(const double* params, int32_t batch, int32_t count,
                                 int32_t padded, const float* mean, const float* inv_std,
                                 uint16_t* out);
+/* The same of two arrays side by side, [batch][first_count] and
+ * [batch][second_count] (a flow instance's supplies and costs), without a
+ * concatenated copy. */
+int32_t pdlpgpu_encode_feature_pair(const double* first, int32_t first_count, const double* second,
+                                    int32_t second_count, int32_t batch, int32_t padded,
+                                    const float* mean, const float* inv_std, uint16_t* out);
 int32_t pdlpgpu_encode_targets(const double* primal, const double* dual, const double* weight,
                                int32_t batch, int32_t n, int32_t m, int32_t out_width,
                                const double* primal_scale, const float* dual_mean,

@@ -1,386 +1,103 @@
 // mlp.cu -- the learned warm start's network, trained and evaluated with
-// this library's own sm_100a kernels:
+// this library's own sm_100a kernels: the tensor-core products of gemm.cuh
+// with their epilogues, and here what surrounds them -- the fixed-order sums
+// of K splits with the layer's activation, the biases' sums and Adam steps,
+// the codec between LP instances and the network, and the host side.
 //
-//   gemm_tn      C[M][N] = A[M][K] * B[N][K]^T, BF16 operands, FP32
-//                accumulation on the 5th-generation tensor cores: TMA
-//                (cp.async.bulk.tensor, 128-byte swizzle) fills a 3-stage
-//                shared-memory ring, one thread issues tcgen05.mma
-//                (M=128, N=128, K=16) into a TMEM accumulator and commits
-//                each stage back to the producer through mbarriers, and the
-//                epilogue reads TMEM with tcgen05.ld. Two CTAs share an SM,
-//                so one's epilogue overlaps the other's main loop; tiles run
-//                in grouped order for L2 reuse. Optional split-K writes one
-//                FP32 partial per K range.
-//   epilogue     sum of the split-K partials in a fixed order, bias,
-//                ReLU, BF16/FP32 outputs
-//   transpose, loss, ReLU backward, bias gradients, Adam
-//
-// Every mbarrier wait gives up after two seconds of %globaltimer, records an
-// error code and lets the CTA drain its copies, free its TMEM and return, so
-// a fault in the pipeline cannot hang the device.
+// A training step (10 launches, each a programmatic launch after the one
+// before) stores no output, no FP32 output gradient, no weight gradient and
+// no transposed operand: the last layer's product ends in the loss and its
+// gradient, and a weight gradient's product ends in Adam.
 #include "pdlpgpu_mlp.h"
+
+#include "gemm.cuh"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
 #include <random>
 #include <string>
+#include <utility>
 #include <vector>
 
 extern "C" void pdlpgpu_internal_set_error(const char* message);
 
 namespace pdlpgpu_mlp_impl {
 
-using bf16 = __nv_bfloat16;
-
-constexpr int BM = 128;
-constexpr int BN = 128;
-constexpr int BK = 64;                       // 64 BF16 = one 128-byte swizzle row
-constexpr int STAGES = 3;                    // two CTAs per SM (shared memory)
-constexpr int GEMM_THREADS = 128;
-constexpr int STAGE_A_BYTES = BM * BK * 2;   // 16 KiB
-constexpr int STAGE_B_BYTES = BN * BK * 2;   // 16 KiB
-constexpr int GEMM_SMEM = STAGES * (STAGE_A_BYTES + STAGE_B_BYTES) + 1024 /*align*/ + 256 /*barriers*/;
-constexpr int64_t kWaitNs = 2000000000LL;
-
-// ---------------------------------------------------------------------------
-// PTX helpers
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ int64_t gtimer() {
-    int64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t phase) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
-
-// Bounded wait: false (and an error code) after kWaitNs without completion.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int* err, int code) {
-    if (mbar_test(bar, phase)) return true;
-    const int64_t t0 = gtimer();
-    while (true) {
-        if (mbar_test(bar, phase)) return true;
-        if (gtimer() - t0 > kWaitNs) {
-            atomicExch(err, code);
-            return false;
-        }
-    }
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                            int32_t x, int32_t y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-        : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups
-// 1024 bytes apart (SBO), version 1.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((addr >> 4) & 0x3fff);         // start address
-    d |= static_cast<uint64_t>(1) << 16;                      // leading byte offset (16 B; unused)
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;              // stride byte offset
-    d |= static_cast<uint64_t>(1) << 46;                      // descriptor version
-    d |= static_cast<uint64_t>(2) << 61;                      // SWIZZLE_128B
-    return d;
-}
-
-// Instruction descriptor: BF16 x BF16 -> FP32, both K-major, M=128, N=BN.
-constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) |
-                                (static_cast<uint32_t>(BN >> 3) << 17) |
-                                (static_cast<uint32_t>(BM >> 4) << 24);
-
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(a), "l"(b), "r"(kInstrDesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-        "%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-          "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-          "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// ---------------------------------------------------------------------------
-// GEMM: one CTA per (128 x 128 output tile, K range)
-// ---------------------------------------------------------------------------
-struct GemmArgs {
-    int M, N, K;
-    int kblocks_per_split;
-    float* C;                // [splits][M][N]
-    int64_t split_stride;
-    int* err;
-};
-
-__global__ void __launch_bounds__(GEMM_THREADS, 2)
-gemm_tn(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-        GemmArgs a) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sa = smem;
-    uint8_t* sb = smem + STAGES * STAGE_A_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sb + STAGES * STAGE_B_BYTES);
-    uint64_t* full = bars;                    // [STAGES]
-    uint64_t* empty = bars + STAGES;          // [STAGES]
-    uint64_t* done = bars + 2 * STAGES;       // [1]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // Grouped tile order: consecutive CTAs sweep kGroupM row tiles for each
-    // column tile, so the CTAs in flight share their A and B panels in L2.
-    constexpr int kGroupM = 16;
-    const int pid = blockIdx.x + blockIdx.y * gridDim.x;
-    const int per_group = kGroupM * gridDim.y;
-    const int first_m = (pid / per_group) * kGroupM;
-    const int group_m = min(static_cast<int>(gridDim.x) - first_m, kGroupM);
-    const int m0 = (first_m + (pid % per_group) % group_m) * BM;
-    const int n0 = ((pid % per_group) / group_m) * BN;
-    const int total_kb = (a.K + BK - 1) / BK;
-    const int kb0 = blockIdx.z * a.kblocks_per_split;
-    const int kb1 = min(total_kb, kb0 + a.kblocks_per_split);
-    const int nk = max(0, kb1 - kb0);
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&full[s]), 1);
-            mbar_init(smem_u32(&empty[s]), 1);
-        }
-        mbar_init(smem_u32(done), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(BN));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
-
-    // Warp-specialised pipeline. Lane 0 of warp 0 produces: it refills a
-    // stage as soon as the MMAs that read it have completed (`empty`), never
-    // waiting on the MMAs of other stages. Lane 0 of warp 1 consumes: it
-    // waits for a stage's bytes (`full`), issues its four MMAs and commits
-    // the stage back, so the tensor pipe always has the next stage queued.
-    __shared__ int consumed_by_mma;
-    if (threadIdx.x == 0) consumed_by_mma = 0;
-    __syncthreads();
-    int issued = 0;
-    if (warp == 0 && lane == 0 && nk > 0) {
-        const uint32_t tx = STAGE_A_BYTES + STAGE_B_BYTES;
-        for (int i = 0; i < nk; ++i) {
-            const int s = i % STAGES;
-            if (i >= STAGES && !mbar_wait(smem_u32(&empty[s]), ((i / STAGES) - 1) & 1, a.err, 2)) break;
-            const uint32_t fb = smem_u32(&full[s]);
-            mbar_expect_tx(fb, tx);
-            tma_load_2d(smem_u32(sa + s * STAGE_A_BYTES), &map_a, fb, (kb0 + i) * BK, m0);
-            tma_load_2d(smem_u32(sb + s * STAGE_B_BYTES), &map_b, fb, (kb0 + i) * BK, n0);
-            ++issued;
-        }
-    } else if (warp == 1 && lane == 0 && nk > 0) {
-        int i = 0;
-        for (; i < nk; ++i) {
-            const int s = i % STAGES;
-            if (!mbar_wait(smem_u32(&full[s]), (i / STAGES) & 1, a.err, 1)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a_base = smem_u32(sa + s * STAGE_A_BYTES);
-            const uint32_t b_base = smem_u32(sb + s * STAGE_B_BYTES);
-#pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-                // K advances 16 BF16 = 32 bytes inside the 128-byte swizzle row.
-                mma_bf16(tmem, smem_desc(a_base + kk * 32), smem_desc(b_base + kk * 32),
-                         (i > 0 || kk > 0) ? 1u : 0u);
-            }
-            mma_commit(smem_u32(&empty[s]));
-        }
-        consumed_by_mma = i;
-        // Arrives once every MMA issued above has completed.
-        mma_commit(smem_u32(done));
-    }
-    __syncthreads();
-    // After an error, copies the MMA warp never consumed may still be in
-    // flight: the producer waits for them (bounded) before the stage memory
-    // is reused below.
-    if (warp == 0 && lane == 0)
-        for (int i = consumed_by_mma; i < issued; ++i)
-            mbar_wait(smem_u32(&full[i % STAGES]), (i / STAGES) & 1, a.err, 3);
-    bool have = nk > 0;
-    if (have) have = mbar_wait(smem_u32(done), 0, a.err, 4);
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-    // Epilogue: warp w owns TMEM lanes [32w, 32w + 32) = output rows. Each
-    // 32 x 32 block goes through shared memory (the drained stage buffers),
-    // so every store instruction writes 32 consecutive floats of one row.
-    float* tile = reinterpret_cast<float*>(sa) + warp * 32 * 33;
-    const int row0 = m0 + warp * 32;
-    float* cbase = a.C + blockIdx.z * a.split_stride;
-    for (int c0 = 0; c0 < BN; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + c0, r);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = have ? __uint_as_float(r[j]) : 0.0f;
-        __syncwarp();
-        const int col = n0 + c0 + lane;
-        for (int rr = 0; rr < 32; ++rr) {
-            const int row = row0 + rr;
-            if (row < a.M && col < a.N) cbase[static_cast<int64_t>(row) * a.N + col] = tile[rr * 33 + lane];
-        }
-        __syncwarp();
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Elementwise kernels
 // ---------------------------------------------------------------------------
-// out = act(sum_z partial[z] + bias) -> optional FP32 and BF16 copies.
-__global__ void epilogue(const float* partial, int splits, int64_t split_stride, int M, int N,
-                         const float* bias, int relu, float* out_f32, bf16* out_bf16) {
-    const int64_t total = static_cast<int64_t>(M) * N;
-    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        float v = 0.0f;
-        for (int z = 0; z < splits; ++z) v += partial[z * split_stride + t];
-        if (bias) v += bias[t % N];
-        if (relu) v = v > 0.0f ? v : 0.0f;
-        if (out_f32) out_f32[t] = v;
-        if (out_bf16) out_bf16[t] = __float2bfloat16_rn(v);
+// The K splits' partials of four neighbouring elements added in split order
+// (every load is in flight before the first add needs it).
+__device__ __forceinline__ void split_sums(const float* partial, int splits, int64_t stride, int64_t t, float (&v)[4]) {
+    v[0] = v[1] = v[2] = v[3] = 0.0f;
+#pragma unroll 6
+    for (int z = 0; z < splits; ++z) {
+        const float4 p = *reinterpret_cast<const float4*>(partial + z * stride + t);
+        v[0] += p.x;
+        v[1] += p.y;
+        v[2] += p.z;
+        v[3] += p.w;
     }
 }
 
-// dst[c][r] = src[r][c] for a rows x cols BF16 matrix.
-__global__ void transpose_bf16(const bf16* src, bf16* dst, int rows, int cols) {
-    __shared__ bf16 tile[32][33];
-    const int c = blockIdx.x * 32 + threadIdx.x;
-    for (int k = 0; k < 32; k += 8) {
-        const int r = blockIdx.y * 32 + threadIdx.y + k;
-        if (r < rows && c < cols) tile[threadIdx.y + k][threadIdx.x] = src[static_cast<int64_t>(r) * cols + c];
-    }
-    __syncthreads();
-    const int r2 = blockIdx.y * 32 + threadIdx.x;
-    for (int k = 0; k < 32; k += 8) {
-        const int c2 = blockIdx.x * 32 + threadIdx.y + k;
-        if (r2 < rows && c2 < cols) dst[static_cast<int64_t>(c2) * rows + r2] = tile[threadIdx.x][threadIdx.y + k];
-    }
+__device__ __forceinline__ void store_bf16x4(bf16* out, const float (&v)[4]) {
+    uint2 u;
+    u.x = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(v[0]))) |
+          (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(v[1]))) << 16);
+    u.y = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(v[2]))) |
+          (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(v[3]))) << 16);
+    *reinterpret_cast<uint2*>(out) = u;
 }
 
-// d = 2 w_j (out - target) / batch, in FP32 and BF16; per-row loss partials.
-__global__ void loss_grad(const float* out, const float* target, const float* w, int B, int N,
-                          float* d_f32, bf16* d_bf16, float* row_loss) {
-    const int b = blockIdx.x;
-    float acc = 0.0f;
-    for (int j = threadIdx.x; j < N; j += blockDim.x) {
-        const int64_t t = static_cast<int64_t>(b) * N + j;
-        const float e = out[t] - target[t];
-        acc += w[j] * e * e;
-        const float g = 2.0f * w[j] * e / static_cast<float>(B);
-        d_f32[t] = g;
-        d_bf16[t] = __float2bfloat16_rn(g);
-    }
-    __shared__ float red[256];
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) row_loss[b] = red[0] / static_cast<float>(B);
+// h = relu(sum of the splits + bias), BF16. N (the hidden width) is a
+// multiple of 64.
+__global__ void __launch_bounds__(128) hidden_forward(const float* partial, int splits, int64_t stride, int N,
+                                                      const float* bias, bf16* h) {
+    pdl_trigger();
+    pdl_wait();
+    const int64_t t = 4 * (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x);
+    if (t >= stride) return;
+    float v[4];
+    split_sums(partial, splits, stride, t, v);
+    const float4 b = *reinterpret_cast<const float4*>(bias + t % N);
+    v[0] += b.x;
+    v[1] += b.y;
+    v[2] += b.z;
+    v[3] += b.w;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = v[k] > 0.0f ? v[k] : 0.0f;
+    store_bf16x4(h + t, v);
 }
 
-__global__ void sum_rows(const float* row_loss, int B, float* loss) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        float s = 0.0f;
-        for (int b = 0; b < B; ++b) s += row_loss[b];
-        *loss = s;
-    }
+// dZ = (sum of the splits) * (H > 0), FP32 (the bias's sum) and BF16 (the
+// products).
+__global__ void __launch_bounds__(128) hidden_backward(const float* partial, int splits, int64_t stride, const bf16* h,
+                                                       float* dz, bf16* dzh) {
+    pdl_trigger();
+    pdl_wait();
+    const int64_t t = 4 * (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x);
+    if (t >= stride) return;
+    float v[4];
+    split_sums(partial, splits, stride, t, v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = __bfloat162float(h[t + k]) > 0.0f ? v[k] : 0.0f;
+    *reinterpret_cast<float4*>(dz + t) = make_float4(v[0], v[1], v[2], v[3]);
+    store_bf16x4(dzh + t, v);
 }
 
-// dZ = dH * (H > 0) -> FP32 and BF16.
-__global__ void relu_backward(const float* dh, const bf16* h, int64_t total, float* dz_f32, bf16* dz_bf16) {
-    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const float v = __bfloat162float(h[t]) > 0.0f ? dh[t] : 0.0f;
-        dz_f32[t] = v;
-        dz_bf16[t] = __float2bfloat16_rn(v);
-    }
-}
-
-// db[j] = sum_b d[b][j] (rows summed in order).
-__global__ void column_sums(const float* d, int B, int N, float* db) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= N) return;
-    float s = 0.0f;
-    for (int b = 0; b < B; ++b) s += d[static_cast<int64_t>(b) * N + j];
-    db[j] = s;
-}
-
-// Adam (Kingma and Ba, 2015) with bias correction; refreshes the BF16 copy.
-__global__ void adam(float* p, const float* g, float* m, float* v, bf16* p_bf16, int64_t n, float lr,
-                     float b1, float b2, float eps, float c1, float c2) {
-    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n;
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const float gr = g[t];
-        const float mt = b1 * m[t] + (1.0f - b1) * gr;
-        const float vt = b2 * v[t] + (1.0f - b2) * gr * gr;
-        m[t] = mt;
-        v[t] = vt;
-        const float upd = lr * (mt / c1) / (sqrtf(vt / c2) + eps);
-        const float pn = p[t] - upd;
-        p[t] = pn;
-        if (p_bf16) p_bf16[t] = __float2bfloat16_rn(pn);
-    }
+// The bias sums and the loss alone (gradient mode; adam_step does them in a
+// training step).
+__global__ void __launch_bounds__(32) bias_and_loss(BiasArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    bias_and_loss_warp(a, static_cast<int>(blockIdx.x));
 }
 
 __global__ void to_bf16(const float* src, bf16* dst, int64_t n) {
@@ -390,52 +107,84 @@ __global__ void to_bf16(const float* src, bf16* dst, int64_t n) {
 }
 
 // --- codec between LP instances and the network -----------------------------
-// Features: standardised instance parameters, BF16, zero-padded to `padded`.
-__global__ void encode_features(const double* params, int B, int P, int padded, const float* mean,
-                                const float* inv_std, bf16* out) {
-    const int64_t total = static_cast<int64_t>(B) * padded;
-    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t b = t / padded;
-        const int k = static_cast<int>(t - b * padded);
-        float v = 0.0f;
-        if (k < P) v = (static_cast<float>(params[b * P + k]) - mean[k]) * inv_std[k];
-        out[t] = __float2bfloat16_rn(v);
+// One row of the batch per blockIdx.y, blockIdx.x * blockDim.x elements of it
+// at a time, four per thread: no element divides its index, and a thread has
+// four independent loads in flight. HBM-bound (20 bytes an element in, 8 to 12
+// out); the flow family's 256 instances of 22,000 parameters.
+constexpr int kCodecThreads = 256;
+constexpr int kCodecItems = 4;
+inline dim3 codec_grid(int64_t width, int rows) {
+    const int64_t per = kCodecThreads * kCodecItems;
+    return dim3(static_cast<unsigned>((width + per - 1) / per), static_cast<unsigned>(rows < 65535 ? rows : 65535));
+}
+
+// f(b, j) for the CTA's elements j < width of its rows b < B: `load` of all
+// items before `store` of the first.
+template <class Load, class Store>
+__device__ __forceinline__ void codec_rows(int B, int width, Load load, Store store) {
+    const int j0 = blockIdx.x * (kCodecThreads * kCodecItems) + threadIdx.x;
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {
+        decltype(load(0, 0)) v[kCodecItems];
+#pragma unroll
+        for (int k = 0; k < kCodecItems; ++k)
+            if (j0 + k * kCodecThreads < width) v[k] = load(b, j0 + k * kCodecThreads);
+#pragma unroll
+        for (int k = 0; k < kCodecItems; ++k)
+            if (j0 + k * kCodecThreads < width) store(b, j0 + k * kCodecThreads, v[k]);
     }
 }
 
+// Features: standardised instance parameters, BF16, zero-padded to `padded`.
+// The parameters are the P of `first` and the Q of `second`, in that order
+// (one array has Q = 0).
+__global__ void __launch_bounds__(kCodecThreads)
+encode_features(const double* first, int P, const double* second, int Q, int B, int padded, const float* mean,
+                const float* inv_std, bf16* out) {
+    codec_rows(
+        B, padded,
+        [&](int b, int k) {
+            const int64_t r = b;
+            if (k >= P + Q) return 0.0f;
+            const double x = k < P ? first[r * P + k] : second[r * Q + (k - P)];
+            return (static_cast<float>(x) - mean[k]) * inv_std[k];
+        },
+        [&](int b, int k, float v) { out[static_cast<int64_t>(b) * padded + k] = __float2bfloat16_rn(v); });
+}
+
 // Targets: primal / scale, standardised dual, standardised log weight, zeros.
-__global__ void encode_targets(const double* x, const double* y, const double* w, int B, int n, int m,
-                               int O, const double* scale, const float* ymean, const float* yinv,
-                               float wmean, float winv, float* out) {
-    const int64_t total = static_cast<int64_t>(B) * O;
-    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t b = t / O;
-        const int j = static_cast<int>(t - b * O);
-        float v = 0.0f;
-        if (j < n) v = static_cast<float>(x[b * n + j] / scale[j]);
-        else if (j < n + m) v = (static_cast<float>(y[b * m + (j - n)]) - ymean[j - n]) * yinv[j - n];
-        else if (j == n + m) v = (logf(static_cast<float>(w[b])) - wmean) * winv;
-        out[t] = v;
-    }
+__global__ void __launch_bounds__(kCodecThreads)
+encode_targets(const double* x, const double* y, const double* w, int B, int n, int m, int O, const double* scale,
+               const float* ymean, const float* yinv, float wmean, float winv, float* out) {
+    codec_rows(
+        B, O,
+        [&](int b, int j) {
+            const int64_t r = b;
+            if (j < n) return static_cast<float>(x[r * n + j] / scale[j]);
+            if (j < n + m) return (static_cast<float>(y[r * m + (j - n)]) - ymean[j - n]) * yinv[j - n];
+            return j == n + m ? (logf(static_cast<float>(w[b])) - wmean) * winv : 0.0f;
+        },
+        [&](int b, int j, float v) { out[static_cast<int64_t>(b) * O + j] = v; });
 }
 
 // Warm start from network outputs: x = clamp(out, 0, 1) * scale, y and the
 // weight de-standardised.
-__global__ void decode_warmstart(const float* out, int B, int n, int m, int O, const double* scale,
-                                 const float* ymean, const float* ystd, float wmean, float wstd,
-                                 double* wx, double* wy, double* ww) {
-    const int64_t total = static_cast<int64_t>(B) * (n + m + 1);
-    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < total;
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int64_t b = t / (n + m + 1);
-        const int j = static_cast<int>(t - b * (n + m + 1));
-        const float v = out[b * O + j];
-        if (j < n) wx[b * n + j] = static_cast<double>(fminf(fmaxf(v, 0.0f), 1.0f)) * scale[j];
-        else if (j < n + m) wy[b * m + (j - n)] = static_cast<double>(v * ystd[j - n] + ymean[j - n]);
-        else ww[b] = static_cast<double>(expf(v * wstd + wmean));
-    }
+__global__ void __launch_bounds__(kCodecThreads)
+decode_warmstart(const float* out, int B, int n, int m, int O, const double* scale, const float* ymean,
+                 const float* ystd, float wmean, float wstd, double* wx, double* wy, double* ww) {
+    codec_rows(
+        B, n + m + 1,
+        [&](int b, int j) {
+            const float v = out[static_cast<int64_t>(b) * O + j];
+            if (j < n) return static_cast<double>(fminf(fmaxf(v, 0.0f), 1.0f)) * scale[j];
+            if (j < n + m) return static_cast<double>(v * ystd[j - n] + ymean[j - n]);
+            return static_cast<double>(expf(v * wstd + wmean));
+        },
+        [&](int b, int j, double v) {
+            const int64_t r = b;
+            if (j < n) wx[r * n + j] = v;
+            else if (j < n + m) wy[r * m + (j - n)] = v;
+            else ww[b] = v;
+        });
 }
 
 inline unsigned grid_for(int64_t n) {
@@ -463,22 +212,25 @@ bool encoder(std::string& err) {
     return true;
 }
 
-// 2-D BF16 row-major [rows][cols] tensor map with a (BK x box_rows) box.
-bool make_map(CUtensorMap& map, const void* base, int64_t rows, int64_t cols, int box_rows,
+// 2-D row-major [rows][cols] tensor map with boxes of box_rows x box_cols,
+// swizzled over the box's rows of 64 or 128 bytes.
+template <class T>
+bool make_map(CUtensorMap& map, const T* base, int64_t rows, int64_t cols, int box_cols, int box_rows,
               std::string& err) {
     if (!encoder(err)) return false;
-    if ((cols * 2) % 16 != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0) {
+    if ((cols * sizeof(T)) % 16 != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0) {
         err = "GEMM operand rows must be 16-byte multiples and 16-byte aligned";
         return false;
     }
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols * 2)};
-    const cuuint32_t box[2] = {static_cast<cuuint32_t>(BK), static_cast<cuuint32_t>(box_rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols * sizeof(T))};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = g_encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims,
-                                strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r =
+        g_encode(&map, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                 const_cast<T*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                 box_cols * sizeof(T) == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         err = "cuTensorMapEncodeTiled failed";
         return false;
@@ -486,46 +238,198 @@ bool make_map(CUtensorMap& map, const void* base, int64_t rows, int64_t cols, in
     return true;
 }
 
-struct GemmLaunch {
-    int splits = 1;
-};
+// An operand of `rows` tile rows over K: stored [rows][K], or [K][rows]
+// (kMn), which is read in boxes of 64 rows x 64 K.
+template <bool kMn>
+bool operand_map(CUtensorMap& map, const bf16* base, int rows, int K, int tile_rows, std::string& err) {
+    return kMn ? make_map(map, base, K, rows, BK, BK, err) : make_map(map, base, rows, K, BK, tile_rows, err);
+}
 
-// C[splits][M][N] partials of A[M][K] * B[N][K]^T.
-bool gemm(const bf16* A, const bf16* B, float* C, int M, int N, int K, int splits, int* err,
-          cudaStream_t s, std::string& msg) {
-    if (M <= 0 || N <= 0 || K <= 0) return true;
+// A kernel's dynamic shared memory limit, set once per device it runs on.
+bool allow_smem(const void* kernel, int bytes, bool (&done)[64], std::string& msg) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (done[dev & 63]) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+        msg = "cudaFuncSetAttribute failed";
+        return false;
+    }
+    done[dev & 63] = true;
+    return true;
+}
+
+// A launch; `after`: it may start while the previous kernel of the stream
+// finishes (the kernel waits for it). cluster_x > 1: clusters along x.
+template <class... P, class... A>
+bool launch(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, bool after, int cluster_x,
+            A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (after) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster_x > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(cluster_x);
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...) == cudaSuccess;
+}
+
+struct Splits {
+    int count, per;   // splits that hold K blocks, K blocks of each (the last may be short)
+};
+Splits effective_splits(int K, int splits) {
+    const int total_kb = (K + BK - 1) / BK;
+    const int asked = std::max(1, std::min(splits, total_kb));
+    const int per = (total_kb + asked - 1) / asked;
+    return {(total_kb + per - 1) / per, per};
+}
+
+// gemm_tile over the whole product: `parallel` runs the splits side by side
+// (one partial each), else every CTA runs its tile's splits one after another.
+template <int kBN, int kStages, bool kAMn, bool kBMn, class Epi>
+bool tile_gemm(const bf16* A, const bf16* B, int M, int N, int K, Splits sp, bool parallel, const Epi& epi, int* err,
+               cudaStream_t s, bool after, std::string& msg) {
+    static bool smem_set[64] = {false};
+    constexpr int smem = tile_smem<kBN, kStages>();
+    auto* kernel = gemm_tile<kBN, kStages, kAMn, kBMn, Epi>;
+    if (!allow_smem(reinterpret_cast<const void*>(kernel), smem, smem_set, msg)) return false;
+    CUtensorMap ma, mb;
+    if (!operand_map<kAMn>(ma, A, M, K, BM, msg) || !operand_map<kBMn>(mb, B, N, K, kBN, msg)) return false;
+    const TileArgs ta{M, N, K, sp.per, parallel ? 1 : sp.count, err};
+    const dim3 grid((M + BM - 1) / BM, (N + kBN - 1) / kBN, parallel ? sp.count : 1);
+    if (!launch(kernel, grid, kTileThreads, smem, s, after, 1, ma, mb, ta, epi)) {
+        msg = "GEMM launch failed";
+        return false;
+    }
+    return true;
+}
+
+// C = A B^T for the two entry points below, without scratch in device memory.
+// The rule, with times in us of the kernels that meet at each line:
+//   one split, at least 56 tiles of 256 x 256 and 1792 tile x K-block steps:
+//     gemm_pair (4096 x 2048 x 4096: 51, gemm_tile 63; 2048^3 21, 21;
+//     4096 x 2048 x 512, below the line: 21 against 19)
+//   several splits on few 128 x 128 tiles: gemm_split, as long as a tile's
+//     CTA would otherwise run long alone (600 x 600 x 8000 in 8 splits: 43 in
+//     one CTA a tile; 300 x 2000 x 8000 in 3, above the line: 35)
+//   else gemm_tile, each CTA its tile's splits in turn: six stages and an SM
+//     to itself while the tiles fit the SMs once or a tile has several splits
+//     to keep apart in TMEM (3000 x 2000 x 4096 in 8: 88, with three stages
+//     184), else three stages and two CTAs an SM (2560 x 1024 x 1024, 160
+//     tiles: 14, with six 19).
+constexpr int64_t kPairMinTiles = 56;
+constexpr int64_t kPairMinSteps = 1792;
+constexpr int64_t kSplitMaxTiles = 40;
+
+bool plain_gemm(const bf16* A, const bf16* B, float* C, int M, int N, int K, int splits, int* err, cudaStream_t s,
+                std::string& msg) {
     if (K % 8 != 0) {
         msg = "GEMM K must be a multiple of 8";
         return false;
     }
-    static bool attr_set[64] = {false};
-    int dev = 0;
+    const Splits sp = effective_splits(K, splits);
+    const int64_t pair_tiles = int64_t((M + 255) / 256) * ((N + 255) / 256);
+    const int64_t tiles = int64_t((M + BM - 1) / BM) * ((N + 127) / 128);
+    int dev = 0, sms = 148;
     cudaGetDevice(&dev);
-    if (!attr_set[dev & 63]) {
-        if (cudaFuncSetAttribute(gemm_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess) {
-            msg = "cudaFuncSetAttribute failed";
-            return false;
-        }
-        attr_set[dev & 63] = true;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sp.count == 1 && pair_tiles >= kPairMinTiles && pair_tiles * ((K + BK - 1) / BK) >= kPairMinSteps) {
+        static bool smem_set[64] = {false};
+        if (!allow_smem(reinterpret_cast<const void*>(gemm_pair), kPairSmem, smem_set, msg)) return false;
+        CUtensorMap ma, mb;
+        if (!make_map(ma, A, M, K, BK, BM, msg) || !make_map(mb, B, N, K, BK, BM, msg)) return false;
+        const PairArgs pa{M, N, K, C, err};
+        const unsigned pairs = static_cast<unsigned>(std::min<int64_t>(pair_tiles, sms / 2));
+        return launch(gemm_pair, dim3(2 * pairs), kPairThreads, kPairSmem, s, false, 1, ma, mb, pa);
     }
-    CUtensorMap ma, mb;
-    if (!make_map(ma, A, M, K, BM, msg) || !make_map(mb, B, N, K, BN, msg)) return false;
-    const int total_kb = (K + BK - 1) / BK;
-    splits = std::max(1, std::min(splits, total_kb));
-    const int per = (total_kb + splits - 1) / splits;
-    splits = (total_kb + per - 1) / per;
-    GemmArgs ga{M, N, K, per, C, static_cast<int64_t>(M) * N, err};
-    dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, splits);
-    gemm_tn<<<grid, GEMM_THREADS, GEMM_SMEM, s>>>(ma, mb, ga);
-    return cudaGetLastError() == cudaSuccess;
+    if (sp.count > 1 && sp.count <= kSplitRanks * kSplitAccs && tiles < kSplitMaxTiles) {
+        static bool smem_set[64] = {false};
+        if (!allow_smem(reinterpret_cast<const void*>(gemm_split), kSplitSmem, smem_set, msg)) return false;
+        CUtensorMap ma, mb;
+        if (!make_map(ma, A, M, K, BK, BM, msg) || !make_map(mb, B, N, K, BK, 128, msg)) return false;
+        // The cluster: as many of the splits side by side as the SMs hold,
+        // and no more accumulators in a CTA than TMEM does.
+        int log_ranks = 1;
+        while ((1 << log_ranks) < kSplitRanks && (2 << log_ranks) <= sp.count &&
+               ((2 * tiles) << log_ranks) <= sms)
+            ++log_ranks;
+        while ((kSplitAccs << log_ranks) < sp.count) ++log_ranks;
+        const TileArgs ta{M, N, K, sp.per, sp.count, err};
+        return launch(gemm_split, dim3(static_cast<unsigned>(tiles << log_ranks)), kTileThreads, kSplitSmem, s, false,
+                      1 << log_ranks, ma, mb, ta, log_ranks, C);
+    }
+    const EpiStore epi{C, 0, nullptr};
+    if (tiles <= sms || sp.count > 1)
+        return tile_gemm<128, 6, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
+    return tile_gemm<128, 3, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
 }
 
 int splits_for(int M, int N, int K) {
-    const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    const int tiles = ((M + BM - 1) / BM) * ((N + 127) / 128);
     const int kb = (K + BK - 1) / BK;
     int s = std::max(1, 148 / std::max(1, tiles));
     return std::min(s, std::max(1, kb / 4));
 }
+
+// Error words of calls that have no model to keep one: a slot of this
+// static array per call in flight, so calls of several threads do not see
+// one another's errors. A slot is zero whenever it is free.
+constexpr int kErrSlots = 64;
+__device__ int g_gemm_err[kErrSlots];
+std::mutex g_err_mutex;
+uint64_t g_err_used = 0;
+
+struct ErrSlot {
+    int slot = -1;
+    int* address = nullptr;
+    bool owned = false;   // all slots taken: an allocation of its own
+    ErrSlot() {
+        {
+            std::lock_guard<std::mutex> lock(g_err_mutex);
+            for (int k = 0; k < kErrSlots && slot < 0; ++k)
+                if (!((g_err_used >> k) & 1)) {
+                    g_err_used |= uint64_t(1) << k;
+                    slot = k;
+                }
+        }
+        void* base = nullptr;
+        if (slot >= 0) {
+            if (cudaGetSymbolAddress(&base, g_gemm_err) == cudaSuccess) address = static_cast<int*>(base) + slot;
+        } else if (cudaMalloc(&base, sizeof(int)) == cudaSuccess) {
+            address = static_cast<int*>(base);
+            owned = true;
+            cudaMemset(address, 0, sizeof(int));
+        }
+    }
+    // Waits for the default stream and returns the error word, clearing it;
+    // a negative value is a CUDA error.
+    int take() {
+        int h = 0;
+        if (cudaMemcpy(&h, address, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+        if (h != 0) cudaMemset(address, 0, sizeof(int));
+        return h;
+    }
+    ~ErrSlot() {
+        if (owned) cudaFree(address);
+        if (slot >= 0) {
+            std::lock_guard<std::mutex> lock(g_err_mutex);
+            g_err_used &= ~(uint64_t(1) << slot);
+        }
+    }
+    ErrSlot(const ErrSlot&) = delete;
+    ErrSlot& operator=(const ErrSlot&) = delete;
+};
 
 }  // namespace pdlpgpu_mlp_impl
 
@@ -533,6 +437,7 @@ using namespace pdlpgpu_mlp_impl;
 
 struct pdlpgpu_mlp {
     int in = 0, hidden = 0, out = 0, batch = 0, device = 0;
+    int sms = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t caller_done = nullptr;
     std::vector<void*> allocs;
@@ -540,23 +445,27 @@ struct pdlpgpu_mlp {
     float *W1 = nullptr, *b1 = nullptr, *W2 = nullptr, *b2 = nullptr, *W3 = nullptr, *b3 = nullptr;
     bf16 *W1h = nullptr, *W2h = nullptr, *W3h = nullptr;
     float *mW1, *vW1, *mb1, *vb1, *mW2, *vW2, *mb2, *vb2, *mW3, *vW3, *mb3, *vb3;
-    float *gW1, *gb1, *gW2, *gb2, *gW3, *gb3;
     // activations and scratch
     bf16 *H1 = nullptr, *H2 = nullptr;
-    float *Out = nullptr, *dOut = nullptr, *dH = nullptr, *dZ = nullptr;
-    bf16 *dOuth, *dZh;
-    bf16 *T1, *T2;              // transposes
-    float* partial = nullptr;   // split-K partials
-    int64_t partial_elems = 0;
-    float* row_loss = nullptr;
-    float* loss_dev = nullptr;
-    int* err = nullptr;
+    float *dZ1 = nullptr, *dZ2 = nullptr;
+    bf16 *dOuth = nullptr, *dZ1h = nullptr, *dZ2h = nullptr;
+    float* partial = nullptr;   // split-K partials of a [batch][hidden] product
+    double* loss_part = nullptr;
+    // What a call reports, read back in one copy: the loss and the pipeline's
+    // error word; `report` is its pinned host copy.
+    struct Report {
+        float loss;
+        int err;
+    };
+    Report *report_dev = nullptr, *report = nullptr;
+    int* err = nullptr;         // &report_dev->err
     int64_t step = 0;
     int64_t launches = 0;
     std::string msg;
 
     ~pdlpgpu_mlp() {
         for (void* p : allocs) cudaFree(p);
+        if (report) cudaFreeHost(report);
         if (caller_done) cudaEventDestroy(caller_done);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -587,102 +496,158 @@ struct pdlpgpu_mlp {
         return true;
     }
 
-    bool run_gemm(const bf16* A, const bf16* B, int M, int N, int K, int splits) {
+    // A launch after the previous one of the call (the call's first is
+    // ordered after the caller's work instead, see wait_for_caller).
+    template <class... P, class... A>
+    bool enqueue(void (*kernel)(P...), int grid, int threads, A&&... args) {
+        const bool after = launches++ > 0;
+        if (launch(kernel, dim3(static_cast<unsigned>(grid)), threads, 0, stream, after, 1, std::forward<A>(args)...))
+            return true;
+        msg = "launch failed";
+        return false;
+    }
+
+    template <int kStages, bool kAMn, bool kBMn, class Epi>
+    bool product(const bf16* A, const bf16* B, int M, int N, int K, Splits sp, const Epi& epi) {
+        const bool after = launches++ > 0;
+        return tile_gemm<128, kStages, kAMn, kBMn>(A, B, M, N, K, sp, true, epi, err, stream, after, msg);
+    }
+
+    // partial[z] of a [batch][hidden] product over K, and its splits. With at
+    // most one CTA per SM the ring is six stages deep (the copies in flight
+    // bound a long K): 22,000 inputs, 512 wide, batch 256.
+    template <bool kBMn>
+    bool hidden_product(const bf16* A, const bf16* B, int K, Splits& sp) {
+        sp = effective_splits(K, splits_for(batch, hidden, K));
+        const EpiStore epi{partial, int64_t(batch) * hidden, nullptr};
+        return product<6, false, kBMn>(A, B, batch, hidden, K, sp, epi);
+    }
+
+    int hidden_ctas() const { return static_cast<int>((int64_t(batch) * hidden / 4 + 127) / 128); }
+
+    bool forward_hidden(const bf16* X) {
+        const int64_t BH = int64_t(batch) * hidden;
+        Splits sp;
+        return hidden_product<false>(X, W1h, in, sp) &&
+               enqueue(hidden_forward, hidden_ctas(), 128, partial, sp.count, BH, hidden, b1, H1) &&
+               hidden_product<false>(H1, W2h, hidden, sp) &&
+               enqueue(hidden_forward, hidden_ctas(), 128, partial, sp.count, BH, hidden, b2, H2);
+    }
+
+    // The last layer's column tile: the whole width over the SMs, in
+    // 32-column blocks, at most 256 columns (one MMA).
+    int last_bn() const { return std::min(256, ((out + sms - 1) / sms + 31) / 32 * 32); }
+    int last_ctas() const { return (out + last_bn() - 1) / last_bn(); }
+
+    template <bool kTrain>
+    bool last(LastArgs la) {
+        const int bn = last_bn();
+        const Splits sp = effective_splits(hidden, std::min(splits_for(batch, out, hidden), kLastTmem / bn));
+        la.M = batch;
+        la.N = out;
+        la.K = hidden;
+        la.bn = bn;
+        la.kb_per_split = sp.per;
+        la.splits = sp.count;
+        la.bias = b3;
+        la.err = err;
+        static bool smem_set[64] = {false};
+        if (!allow_smem(reinterpret_cast<const void*>(last_layer<kTrain>), last_smem(256), smem_set, msg)) return false;
+        CUtensorMap ma, mb;
+        if (!make_map(ma, H2, batch, hidden, BK, BM, msg) || !make_map(mb, W3h, out, hidden, BK, bn, msg)) return false;
         ++launches;
-        return gemm(A, B, partial, M, N, K, splits, err, stream, msg);
+        if (launch(last_layer<kTrain>, dim3(static_cast<unsigned>(last_ctas())), kLastThreads, last_smem(bn), stream, true,
+                   1, ma, mb, la))
+            return true;
+        msg = "GEMM launch failed";
+        return false;
     }
 
-    void finish(int M, int N, int splits, const float* bias, int relu, float* of, bf16* ob) {
-        epilogue<<<grid_for(static_cast<int64_t>(M) * N), 256, 0, stream>>>(
-            partial, splits, static_cast<int64_t>(M) * N, M, N, bias, relu, of, ob);
-        ++launches;
+    bool forward(const bf16* X, float* outputs) {
+        LastArgs la{};
+        la.out = outputs;
+        return forward_hidden(X) && last<false>(la);
     }
 
-    void transpose(const bf16* src, bf16* dst, int rows, int cols) {
-        dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
-        transpose_bf16<<<grid, block, 0, stream>>>(src, dst, rows, cols);
-        ++launches;
+    // Gradients wanted by the caller (any may be null), or, when `lr` is not
+    // negative, an Adam step.
+    struct Gradients {
+        float *W1 = nullptr, *b1 = nullptr, *W2 = nullptr, *b2 = nullptr, *W3 = nullptr, *b3 = nullptr;
+    };
+
+    // dW = D^T A of a [batch][rows] and a [batch][cols] matrix, both operands
+    // as they lie, into `grad`.
+    bool weight_gradient(const bf16* D, const bf16* A, int rows, int cols, float* grad) {
+        return grad == nullptr || product<3, true, true>(D, A, rows, cols, batch, effective_splits(batch, 1),
+                                                         EpiStore{grad, 0, nullptr});
+    }
+    bool adam_layer(AdamLayer& L, const bf16* D, const bf16* A, int rows, int cols, float* p, float* m, float* v,
+                    bf16* h) {
+        L.rows = rows;
+        L.cols = cols;
+        L.tiles_n = (cols + kAdamBN - 1) / kAdamBN;
+        L.tiles = (rows + BM - 1) / BM * L.tiles_n;
+        return operand_map<true>(L.d, D, rows, batch, BM, msg) && operand_map<true>(L.a, A, cols, batch, kAdamBN, msg) &&
+               make_map(L.p, p, rows, cols, 32, BM, msg) && make_map(L.m, m, rows, cols, 32, BM, msg) &&
+               make_map(L.v, v, rows, cols, 32, BM, msg) && make_map(L.h, h, rows, cols, 32, BM, msg);
     }
 
-    int effective_splits(int M, int N, int K) const {
-        const int total_kb = (K + BK - 1) / BK;
-        int s = std::max(1, std::min(splits_for(M, N, K), total_kb));
-        const int per = (total_kb + s - 1) / s;
-        return (total_kb + per - 1) / per;
-    }
-
-    bool forward(const bf16* X) {
-        const int B = batch;
-        int s = effective_splits(B, hidden, in);
-        if (!run_gemm(X, W1h, B, hidden, in, s)) return false;
-        finish(B, hidden, s, b1, 1, nullptr, H1);
-        s = effective_splits(B, hidden, hidden);
-        if (!run_gemm(H1, W2h, B, hidden, hidden, s)) return false;
-        finish(B, hidden, s, b2, 1, nullptr, H2);
-        s = effective_splits(B, out, hidden);
-        if (!run_gemm(H2, W3h, B, out, hidden, s)) return false;
-        finish(B, out, s, b3, 0, Out, nullptr);
-        return true;
-    }
-
-    bool backward(const bf16* X, const float* target, const float* w) {
-        const int B = batch;
-        loss_grad<<<B, 256, 0, stream>>>(Out, target, w, B, out, dOut, dOuth, row_loss);
-        sum_rows<<<1, 32, 0, stream>>>(row_loss, B, loss_dev);
-        column_sums<<<(out + 255) / 256, 256, 0, stream>>>(dOut, B, out, gb3);
-        launches += 3;
-        // dW3 = dOut^T H2
-        transpose(dOuth, T1, B, out);        // [out][B]
-        transpose(H2, T2, B, hidden);        // [hidden][B]
-        if (!run_gemm(T1, T2, out, hidden, B, 1)) return false;
-        finish(out, hidden, 1, nullptr, 0, gW3, nullptr);
-        // dH2 = dOut W3 = dOut (W3^T)^T
-        transpose(W3h, T1, out, hidden);     // [hidden][out]
-        int s = effective_splits(B, hidden, out);
-        if (!run_gemm(dOuth, T1, B, hidden, out, s)) return false;
-        finish(B, hidden, s, nullptr, 0, dH, nullptr);
-        relu_backward<<<grid_for(static_cast<int64_t>(B) * hidden), 256, 0, stream>>>(
-            dH, H2, static_cast<int64_t>(B) * hidden, dZ, dZh);
-        column_sums<<<(hidden + 255) / 256, 256, 0, stream>>>(dZ, B, hidden, gb2);
-        launches += 2;
-        // dW2 = dZ2^T H1
-        transpose(dZh, T1, B, hidden);
-        transpose(H1, T2, B, hidden);
-        if (!run_gemm(T1, T2, hidden, hidden, B, 1)) return false;
-        finish(hidden, hidden, 1, nullptr, 0, gW2, nullptr);
-        // dH1 = dZ2 W2
-        transpose(W2h, T1, hidden, hidden);
-        s = effective_splits(B, hidden, hidden);
-        if (!run_gemm(dZh, T1, B, hidden, hidden, s)) return false;
-        finish(B, hidden, s, nullptr, 0, dH, nullptr);
-        relu_backward<<<grid_for(static_cast<int64_t>(B) * hidden), 256, 0, stream>>>(
-            dH, H1, static_cast<int64_t>(B) * hidden, dZ, dZh);
-        column_sums<<<(hidden + 255) / 256, 256, 0, stream>>>(dZ, B, hidden, gb1);
-        launches += 2;
-        // dW1 = dZ1^T X
-        transpose(dZh, T1, B, hidden);
-        transpose(X, T2, B, in);             // [in][B]
-        if (!run_gemm(T1, T2, hidden, in, B, 1)) return false;
-        finish(hidden, in, 1, nullptr, 0, gW1, nullptr);
-        return true;
-    }
-
-    void adam_all(float lr) {
-        ++step;
-        const float b1c = 0.9f, b2c = 0.999f, eps = 1e-8f;
-        const float c1 = 1.0f - std::pow(b1c, static_cast<float>(step));
-        const float c2 = 1.0f - std::pow(b2c, static_cast<float>(step));
-        struct P { float* p; float* g; float* m; float* v; bf16* h; int64_t n; };
-        const P ps[6] = {{W1, gW1, mW1, vW1, W1h, int64_t(hidden) * in},
-                         {b1, gb1, mb1, vb1, nullptr, hidden},
-                         {W2, gW2, mW2, vW2, W2h, int64_t(hidden) * hidden},
-                         {b2, gb2, mb2, vb2, nullptr, hidden},
-                         {W3, gW3, mW3, vW3, W3h, int64_t(out) * hidden},
-                         {b3, gb3, mb3, vb3, nullptr, out}};
-        for (const P& q : ps) {
-            adam<<<grid_for(q.n), 256, 0, stream>>>(q.p, q.g, q.m, q.v, q.h, q.n, lr, b1c, b2c, eps, c1, c2);
-            ++launches;
+    bool step_or_gradients(const bf16* X, const float* target, const float* w, bool train, float lr,
+                           const Gradients& g) {
+        AdamStep adam{lr, 0.9f, 0.999f, 1e-8f, 1.0f, 1.0f, 1.0f, 1.0f};
+        if (train) {
+            ++step;
+            adam.c1 = 1.0f - std::pow(adam.b1, static_cast<float>(step));
+            adam.c2 = 1.0f - std::pow(adam.b2, static_cast<float>(step));
+            adam.r1 = 1.0f / adam.c1;
+            adam.r2 = 1.0f / adam.c2;
         }
+        LastArgs la{};
+        la.target = target;
+        la.weight = w;
+        la.d = dOuth;
+        la.loss_part = loss_part;
+        // In gradient mode the bias gradient always has a place to go: the
+        // split-K partials are free while the last layer runs.
+        la.gb = train ? nullptr : (g.b3 != nullptr ? g.b3 : partial);
+        la.mb = mb3;
+        la.vb = vb3;
+        la.adam = adam;
+        if (!forward_hidden(X) || !last<true>(la)) return false;
+        // dH2 = dOut W3 and dH1 = dZ2 W2 read the weights as they are stored
+        // (K x hidden), before the Adam steps below change them.
+        const int64_t BH = int64_t(batch) * hidden;
+        Splits sp;
+        if (!hidden_product<true>(dOuth, W3h, out, sp) ||
+            !enqueue(hidden_backward, hidden_ctas(), 128, partial, sp.count, BH, H2, dZ2, dZ2h) ||
+            !hidden_product<true>(dZ2h, W2h, hidden, sp) ||
+            !enqueue(hidden_backward, hidden_ctas(), 128, partial, sp.count, BH, H1, dZ1, dZ1h))
+            return false;
+        const BiasArgs ba{{dZ1, dZ2}, {b1, b2}, {mb1, mb2}, {vb1, vb2}, {g.b1, g.b2}, batch, hidden, !train, adam,
+                          loss_part, last_ctas(), &report_dev->loss};
+        if (!train)
+            return weight_gradient(dOuth, H2, out, hidden, g.W3) && weight_gradient(dZ1h, X, hidden, in, g.W1) &&
+                   weight_gradient(dZ2h, H1, hidden, hidden, g.W2) &&
+                   enqueue(bias_and_loss, bias_warps(hidden), 32, ba);
+        AdamArgs aa;
+        if (!adam_layer(aa.layer[0], dZ2h, H1, hidden, hidden, W2, mW2, vW2, W2h) ||
+            !adam_layer(aa.layer[1], dOuth, H2, out, hidden, W3, mW3, vW3, W3h) ||
+            !adam_layer(aa.layer[2], dZ1h, X, hidden, in, W1, mW1, vW1, W1h))
+            return false;
+        aa.adam = adam;
+        aa.bias = ba;
+        aa.K = batch;
+        aa.tiles = aa.layer[0].tiles + aa.layer[1].tiles + aa.layer[2].tiles;
+        aa.err = err;
+        static bool smem_set[64] = {false};
+        if (!allow_smem(reinterpret_cast<const void*>(adam_step), kAdamSmem, smem_set, msg)) return false;
+        ++launches;
+        if (!launch(adam_step, dim3(static_cast<unsigned>(std::min(aa.tiles, sms))), kAdamThreads, kAdamSmem, stream,
+                    true, 1, aa)) {
+            msg = "Adam launch failed";
+            return false;
+        }
+        return true;
     }
 
     void refresh_bf16() {
@@ -691,15 +656,16 @@ struct pdlpgpu_mlp {
         to_bf16<<<grid_for(int64_t(out) * hidden), 256, 0, stream>>>(W3, W3h, int64_t(out) * hidden);
     }
 
-    bool check_err(const char* what) {
-        int h = 0;
-        if (cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+    // Waits for the call; false on a CUDA error or a pipeline timeout.
+    bool finish(const char* what, float* loss) {
+        if (cudaMemcpyAsync(report, report_dev, sizeof(Report), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
             cudaStreamSynchronize(stream) != cudaSuccess) {
             msg = std::string(what) + ": " + cudaGetErrorString(cudaGetLastError());
             return false;
         }
-        if (h != 0) {
-            msg = std::string(what) + ": tensor-core pipeline wait timed out (code " + std::to_string(h) + ")";
+        if (loss) *loss = report->loss;
+        if (report->err != 0) {
+            msg = std::string(what) + ": tensor-core pipeline wait timed out (code " + std::to_string(report->err) + ")";
             cudaMemsetAsync(err, 0, sizeof(int), stream);
             return false;
         }
@@ -727,24 +693,29 @@ int32_t pdlpgpu_mlp_create(int32_t in, int32_t hidden, int32_t out, int32_t batc
         delete m;
         return fail("mlp: cannot use the device");
     }
+    if (cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) m->sms = 148;
     const int64_t H = hidden, I = in, O = out, B = batch;
     bool ok = m->alloc(m->W1, H * I) && m->alloc(m->b1, H) && m->alloc(m->W2, H * H) &&
               m->alloc(m->b2, H) && m->alloc(m->W3, O * H) && m->alloc(m->b3, O) &&
               m->alloc(m->W1h, H * I) && m->alloc(m->W2h, H * H) && m->alloc(m->W3h, O * H);
-    for (auto* q : {&m->mW1, &m->vW1, &m->gW1}) ok = ok && m->alloc(*q, H * I);
-    for (auto* q : {&m->mW2, &m->vW2, &m->gW2}) ok = ok && m->alloc(*q, H * H);
-    for (auto* q : {&m->mW3, &m->vW3, &m->gW3}) ok = ok && m->alloc(*q, O * H);
-    for (auto* q : {&m->mb1, &m->vb1, &m->gb1, &m->mb2, &m->vb2, &m->gb2}) ok = ok && m->alloc(*q, H);
-    for (auto* q : {&m->mb3, &m->vb3, &m->gb3}) ok = ok && m->alloc(*q, O);
-    const int64_t big = std::max(std::max(B * O, O * H), std::max(H * I, B * I));
-    ok = ok && m->alloc(m->H1, B * H) && m->alloc(m->H2, B * H) && m->alloc(m->Out, B * O) &&
-         m->alloc(m->dOut, B * O) && m->alloc(m->dOuth, B * O) && m->alloc(m->dH, B * H) &&
-         m->alloc(m->dZ, B * H) && m->alloc(m->dZh, B * H) && m->alloc(m->T1, big) &&
-         m->alloc(m->T2, big) && m->alloc(m->row_loss, B) && m->alloc(m->loss_dev, 1) &&
-         m->alloc(m->err, 1);
-    // Split-K partials: the largest split GEMMs are [B x H] with K = in or out.
-    m->partial_elems = std::max<int64_t>(std::max(O * H, H * I), std::max(B * O, 160 * B * H));
-    ok = ok && m->alloc(m->partial, m->partial_elems);
+    for (auto* q : {&m->mW1, &m->vW1}) ok = ok && m->alloc(*q, H * I);
+    for (auto* q : {&m->mW2, &m->vW2}) ok = ok && m->alloc(*q, H * H);
+    for (auto* q : {&m->mW3, &m->vW3}) ok = ok && m->alloc(*q, O * H);
+    for (auto* q : {&m->mb1, &m->vb1, &m->mb2, &m->vb2}) ok = ok && m->alloc(*q, H);
+    for (auto* q : {&m->mb3, &m->vb3}) ok = ok && m->alloc(*q, O);
+    for (auto* q : {&m->H1, &m->H2, &m->dZ1h, &m->dZ2h}) ok = ok && m->alloc(*q, B * H);
+    for (auto* q : {&m->dZ1, &m->dZ2}) ok = ok && m->alloc(*q, B * H);
+    ok = ok && m->alloc(m->dOuth, B * O) && m->alloc(m->loss_part, m->last_ctas()) && m->alloc(m->report_dev, 1);
+    // Split-K partials of the [B x H] products (at least O: see gb in step_or_gradients).
+    int64_t parts = 1;
+    for (int k : {in, hidden, out})
+        parts = std::max<int64_t>(parts, effective_splits(k, splits_for(batch, hidden, k)).count);
+    ok = ok && m->alloc(m->partial, std::max(parts * B * H, O));
+    if (ok && cudaMallocHost(reinterpret_cast<void**>(&m->report), sizeof(pdlpgpu_mlp::Report)) != cudaSuccess) {
+        m->msg = "cudaMallocHost failed";
+        ok = false;
+    }
+    if (ok) m->err = &m->report_dev->err;
     if (!ok) {
         const std::string msg = m->msg;
         delete m;
@@ -778,11 +749,8 @@ int32_t pdlpgpu_mlp_forward(pdlpgpu_mlp* m, const uint16_t* inputs, float* outpu
     cudaSetDevice(m->device);
     m->launches = 0;
     if (!m->wait_for_caller()) return fail("mlp forward: stream wait failed");
-    if (!m->forward(reinterpret_cast<const bf16*>(inputs))) return fail("mlp forward: " + m->msg);
-    if (cudaMemcpyAsync(outputs, m->Out, sizeof(float) * m->batch * m->out, cudaMemcpyDeviceToDevice,
-                        m->stream) != cudaSuccess)
-        return fail("mlp forward: copy failed");
-    if (!m->check_err("mlp forward")) return fail(m->msg);
+    if (!m->forward(reinterpret_cast<const bf16*>(inputs), outputs)) return fail("mlp forward: " + m->msg);
+    if (!m->finish("mlp forward", nullptr)) return fail(m->msg);
     return 0;
 }
 
@@ -793,16 +761,10 @@ int32_t pdlpgpu_mlp_gradients(pdlpgpu_mlp* m, const uint16_t* inputs, const floa
     cudaSetDevice(m->device);
     m->launches = 0;
     if (!m->wait_for_caller()) return fail("mlp gradients: stream wait failed");
-    const bf16* X = reinterpret_cast<const bf16*>(inputs);
-    if (!m->forward(X) || !m->backward(X, targets, w)) return fail("mlp gradients: " + m->msg);
-    const int64_t H = m->hidden, I = m->in, O = m->out;
-    auto cp = [&](float* dst, const float* src, int64_t n) {
-        if (dst) cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyDeviceToDevice, m->stream);
-    };
-    cp(dW1, m->gW1, H * I); cp(db1, m->gb1, H); cp(dW2, m->gW2, H * H); cp(db2, m->gb2, H);
-    cp(dW3, m->gW3, O * H); cp(db3, m->gb3, O);
-    if (loss) cudaMemcpyAsync(loss, m->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, m->stream);
-    if (!m->check_err("mlp gradients")) return fail(m->msg);
+    const pdlpgpu_mlp::Gradients g{dW1, db1, dW2, db2, dW3, db3};
+    if (!m->step_or_gradients(reinterpret_cast<const bf16*>(inputs), targets, w, false, 0.0f, g))
+        return fail("mlp gradients: " + m->msg);
+    if (!m->finish("mlp gradients", loss)) return fail(m->msg);
     return 0;
 }
 
@@ -812,11 +774,9 @@ int32_t pdlpgpu_mlp_train_step(pdlpgpu_mlp* m, const uint16_t* inputs, const flo
     cudaSetDevice(m->device);
     m->launches = 0;
     if (!m->wait_for_caller()) return fail("mlp train: stream wait failed");
-    const bf16* X = reinterpret_cast<const bf16*>(inputs);
-    if (!m->forward(X) || !m->backward(X, targets, w)) return fail("mlp train: " + m->msg);
-    m->adam_all(lr);
-    if (loss) cudaMemcpyAsync(loss, m->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, m->stream);
-    if (!m->check_err("mlp train")) return fail(m->msg);
+    if (!m->step_or_gradients(reinterpret_cast<const bf16*>(inputs), targets, w, true, lr, {}))
+        return fail("mlp train: " + m->msg);
+    if (!m->finish("mlp train", loss)) return fail(m->msg);
     return 0;
 }
 
@@ -853,34 +813,15 @@ int64_t pdlpgpu_mlp_launches(pdlpgpu_mlp* m) { return m ? m->launches : 0; }
 
 int32_t pdlpgpu_gemm_bf16(int32_t M, int32_t N, int32_t K, const uint16_t* A, const uint16_t* B,
                           float* C, int32_t splits) {
-    int* err = nullptr;
-    float* partial = nullptr;
-    std::string msg;
     if (M <= 0 || N <= 0 || K <= 0) return fail("gemm: sizes must be positive");
-    const int total_kb = (K + BK - 1) / BK;
-    splits = std::max(1, std::min(splits, total_kb));
-    const int per = (total_kb + splits - 1) / splits;
-    const int s_eff = (total_kb + per - 1) / per;
-    if (cudaMalloc(&err, sizeof(int)) != cudaSuccess) return fail("gemm: cudaMalloc failed");
-    cudaMemset(err, 0, sizeof(int));
-    if (s_eff > 1 && cudaMalloc(&partial, sizeof(float) * static_cast<size_t>(s_eff) * M * N) != cudaSuccess) {
-        cudaFree(err);
-        return fail("gemm: cudaMalloc failed");
-    }
-    float* target = s_eff > 1 ? partial : C;
-    bool ok = gemm(reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(B), target, M, N, K,
-                   s_eff, err, nullptr, msg);
-    if (ok && s_eff > 1)
-        epilogue<<<grid_for(static_cast<int64_t>(M) * N), 256>>>(partial, s_eff, static_cast<int64_t>(M) * N,
-                                                                  M, N, nullptr, 0, C, nullptr);
-    int h = 0;
-    if (cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) ok = false;
-    if (h != 0) {
-        ok = false;
-        msg = "tensor-core pipeline wait timed out (code " + std::to_string(h) + ")";
-    }
-    cudaFree(err);
-    if (partial) cudaFree(partial);
+    ErrSlot err;
+    if (err.address == nullptr) return fail("gemm: no error word");
+    std::string msg;
+    bool ok = plain_gemm(reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(B), C, M, N, K, splits,
+                         err.address, nullptr, msg);
+    const int h = err.take();
+    if (h > 0) msg = "tensor-core pipeline wait timed out (code " + std::to_string(h) + ")";
+    ok = ok && h == 0;
     return ok ? 0 : fail("gemm: " + (msg.empty() ? std::string(cudaGetErrorString(cudaGetLastError())) : msg));
 }
 
@@ -889,27 +830,12 @@ int32_t pdlpgpu_gemm_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, co
                           float* C, int32_t splits, int32_t reps, double* ms_per_call) {
     if (M <= 0 || N <= 0 || K <= 0 || reps <= 0 || ms_per_call == nullptr)
         return fail("gemm_time: sizes and repetitions must be positive");
-    const int total_kb = (K + BK - 1) / BK;
-    splits = std::max(1, std::min(splits, total_kb));
-    const int per = (total_kb + splits - 1) / splits;
-    const int s_eff = (total_kb + per - 1) / per;
-    int* err = nullptr;
-    float* partial = nullptr;
-    if (cudaMalloc(&err, sizeof(int)) != cudaSuccess) return fail("gemm_time: cudaMalloc failed");
-    cudaMemset(err, 0, sizeof(int));
-    if (s_eff > 1 && cudaMalloc(&partial, sizeof(float) * static_cast<size_t>(s_eff) * M * N) != cudaSuccess) {
-        cudaFree(err);
-        return fail("gemm_time: cudaMalloc failed");
-    }
-    float* target = s_eff > 1 ? partial : C;
+    ErrSlot err;
+    if (err.address == nullptr) return fail("gemm_time: no error word");
     std::string msg;
     auto once = [&]() {
-        bool ok = gemm(reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(B), target, M, N, K,
-                       s_eff, err, nullptr, msg);
-        if (ok && s_eff > 1)
-            epilogue<<<grid_for(static_cast<int64_t>(M) * N), 256>>>(partial, s_eff, static_cast<int64_t>(M) * N,
-                                                                      M, N, nullptr, 0, C, nullptr);
-        return ok;
+        return plain_gemm(reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(B), C, M, N, K, splits,
+                          err.address, nullptr, msg);
     };
     bool ok = once();   // warm-up: tensor maps, instruction cache
     cudaEvent_t e0, e1;
@@ -923,14 +849,9 @@ int32_t pdlpgpu_gemm_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, co
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    int h = 0;
-    if (cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) ok = false;
-    if (h != 0) {
-        ok = false;
-        msg = "tensor-core pipeline wait timed out (code " + std::to_string(h) + ")";
-    }
-    cudaFree(err);
-    if (partial) cudaFree(partial);
+    const int h = err.take();
+    if (h > 0) msg = "tensor-core pipeline wait timed out (code " + std::to_string(h) + ")";
+    ok = ok && h == 0;
     *ms_per_call = ms / reps;
     return ok ? 0 : fail("gemm_time: " + (msg.empty() ? std::string(cudaGetErrorString(cudaGetLastError())) : msg));
 }
@@ -938,9 +859,20 @@ int32_t pdlpgpu_gemm_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, co
 int32_t pdlpgpu_encode_features(const double* params, int32_t batch, int32_t count, int32_t padded,
                                 const float* mean, const float* inv_std, uint16_t* out) {
     if (batch <= 0 || count <= 0 || padded < count) return fail("encode_features: bad sizes");
-    encode_features<<<grid_for(static_cast<int64_t>(batch) * padded), 256>>>(
-        params, batch, count, padded, mean, inv_std, reinterpret_cast<bf16*>(out));
+    encode_features<<<codec_grid(padded, batch), kCodecThreads>>>(
+        params, count, nullptr, 0, batch, padded, mean, inv_std, reinterpret_cast<bf16*>(out));
     return cudaGetLastError() == cudaSuccess ? 0 : fail("encode_features: launch failed");
+}
+
+int32_t pdlpgpu_encode_feature_pair(const double* first, int32_t first_count, const double* second,
+                                    int32_t second_count, int32_t batch, int32_t padded, const float* mean,
+                                    const float* inv_std, uint16_t* out) {
+    const int64_t count = static_cast<int64_t>(first_count) + second_count;
+    if (batch <= 0 || first_count <= 0 || second_count <= 0 || padded < count)
+        return fail("encode_feature_pair: bad sizes");
+    encode_features<<<codec_grid(padded, batch), kCodecThreads>>>(
+        first, first_count, second, second_count, batch, padded, mean, inv_std, reinterpret_cast<bf16*>(out));
+    return cudaGetLastError() == cudaSuccess ? 0 : fail("encode_feature_pair: launch failed");
 }
 
 int32_t pdlpgpu_encode_targets(const double* primal, const double* dual, const double* weight,
@@ -949,7 +881,7 @@ int32_t pdlpgpu_encode_targets(const double* primal, const double* dual, const d
                                const float* dual_inv_std, float weight_mean, float weight_inv_std,
                                float* targets) {
     if (batch <= 0 || out_width < n + m + 1) return fail("encode_targets: bad sizes");
-    encode_targets<<<grid_for(static_cast<int64_t>(batch) * out_width), 256>>>(
+    encode_targets<<<codec_grid(out_width, batch), kCodecThreads>>>(
         primal, dual, weight, batch, n, m, out_width, primal_scale, dual_mean, dual_inv_std,
         weight_mean, weight_inv_std, targets);
     return cudaGetLastError() == cudaSuccess ? 0 : fail("encode_targets: launch failed");
@@ -960,7 +892,7 @@ int32_t pdlpgpu_decode_warmstart(const float* outputs, int32_t batch, int32_t n,
                                  const float* dual_mean, const float* dual_std, float weight_mean,
                                  float weight_std, double* primal, double* dual, double* weight) {
     if (batch <= 0 || out_width < n + m + 1) return fail("decode_warmstart: bad sizes");
-    decode_warmstart<<<grid_for(static_cast<int64_t>(batch) * (n + m + 1)), 256>>>(
+    decode_warmstart<<<codec_grid(static_cast<int64_t>(n) + m + 1, batch), kCodecThreads>>>(
         outputs, batch, n, m, out_width, primal_scale, dual_mean, dual_std, weight_mean, weight_std,
         primal, dual, weight);
     return cudaGetLastError() == cudaSuccess ? 0 : fail("decode_warmstart: launch failed");

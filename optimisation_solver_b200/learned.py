@@ -69,10 +69,20 @@ class FlowWarmStart:
             wmean=float(lw.mean()), wstd=float(max(lw.std(), 1e-3)))
 
     def _features(self, supply_dev, cost_dev, out_bf16):
-        params = self.torch.cat([supply_dev, cost_dev], dim=1).contiguous()
-        rc = native.lib().pdlpgpu_encode_features(_p(params), params.shape[0], self.count,
-                                                  self.padded, _p(self.stats["fmean"]),
-                                                  _p(self.stats["finv"]), _p(out_bf16))
+        t = self.torch
+        rows = supply_dev.shape[0]
+        if all(x.is_cuda and x.dtype == t.float64 and x.is_contiguous() and tuple(x.shape) == (rows, k)
+               for x, k in ((supply_dev, self.m), (cost_dev, self.n))) and rows > 0:
+            # The usual case needs no concatenated copy (45 MB each way for
+            # 256 instances of 22,000 parameters: 18 us of the prediction).
+            rc = native.lib().pdlpgpu_encode_feature_pair(
+                _p(supply_dev), self.m, _p(cost_dev), self.n, rows, self.padded,
+                _p(self.stats["fmean"]), _p(self.stats["finv"]), _p(out_bf16))
+        else:
+            params = t.cat([supply_dev, cost_dev], dim=1).contiguous()
+            rc = native.lib().pdlpgpu_encode_features(_p(params), params.shape[0], self.count,
+                                                      self.padded, _p(self.stats["fmean"]),
+                                                      _p(self.stats["finv"]), _p(out_bf16))
         if rc != 0:
             raise RuntimeError(native.last_error())
 

@@ -179,6 +179,9 @@ SIGNATURES = {
     "pdlpgpu_mlp_launches": (C.c_int64, [C.c_void_p]),
     "pdlpgpu_encode_features": (C.c_int32, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
                                             C.c_void_p, C.c_void_p, C.c_void_p]),
+    "pdlpgpu_encode_feature_pair": (C.c_int32, [C.c_void_p, C.c_int32, C.c_void_p, C.c_int32,
+                                                C.c_int32, C.c_int32, C.c_void_p, C.c_void_p,
+                                                C.c_void_p]),
     "pdlpgpu_encode_targets": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32,
                                            C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p,
                                            C.c_void_p, C.c_float, C.c_float, C.c_void_p]),
