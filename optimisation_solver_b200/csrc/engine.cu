@@ -886,10 +886,8 @@ int Engine::timed_position(int k, int slots) const {
 // Small instances run the trials of a check interval in one cluster launch
 // per precision (k_fused) instead of two launches per trial slot: up to 16
 // instances whose slices' warp sums fit a CTA's shared memory, when the
-// device can hold such a cluster. When the cluster has a warp for every
-// slice and the warps' slices fit beside the sums, the slices are staged in
-// shared memory for the launch, and when x and y fit beside them too, every
-// CTA keeps copies of them and no trial touches global memory.
+// device can hold such a cluster. The layout of the vectors (FusedMode) is the
+// first that fits the shared memory of the launch's working precision.
 void Engine::choose_fused() {
     fused_cluster_ = 0;
     fused_shape32_ = fused_shape64_ = FusedShape{};
@@ -897,41 +895,40 @@ void Engine::choose_fused() {
     // The fused kernel adds an entry's slice sums in slice order; that
     // equals the two-kernel path's block sum (one slice per warp, warps in
     // order) only while no entry has more slices than a CTA has warps.
-    bool multi = false;
     for (const auto* side : {&a_ctas_, &at_ctas_})
-        for (const CtaWork& cw : *side) {
+        for (const CtaWork& cw : *side)
             if (cw.slice_end - cw.slice_begin > kThreads / 32) return;
-            multi = multi || cw.slice_end - cw.slice_begin != 1;
-        }
     // An instance's slices are contiguous in its CTA map.
     auto first = [](const std::vector<CtaWork>& side, int e0) { return side[static_cast<size_t>(e0)].slice_begin; };
     auto last = [](const std::vector<CtaWork>& side, int e1) { return side[static_cast<size_t>(e1 - 1)].slice_end; };
     FusedShape sh{};
-    sh.multi = multi ? 1 : 0;
     sh.elem = static_cast<int32_t>(sizeof(double));
+    int32_t rows = 0, cols_rows = 0;   // most 2 m and 2 m + n of an instance
     for (int b = 0; b < count_; ++b) {
         const InstanceInfo& inf = info_[static_cast<size_t>(b)];
         sh.slices_p = std::max(sh.slices_p, last(at_ctas_, inf.at_cta_end) - first(at_ctas_, inf.at_cta_begin));
         sh.slices_d = std::max(sh.slices_d, last(a_ctas_, inf.a_cta_end) - first(a_ctas_, inf.a_cta_begin));
         sh.entries_p = std::max(sh.entries_p, inf.at_cta_end - inf.at_cta_begin);
         sh.entries_d = std::max(sh.entries_d, inf.a_cta_end - inf.a_cta_begin);
+        rows = std::max<int32_t>(rows, static_cast<int32_t>(std::min<int64_t>(2 * int64_t(inf.m), INT32_MAX)));
+        cols_rows = std::max<int32_t>(
+            cols_rows, static_cast<int32_t>(std::min<int64_t>(2 * int64_t(inf.m) + inf.n, INT32_MAX)));
     }
     if (fused_smem_bytes(sh) > kFusedMaxSmemHost) return;
-    const int warps_per_cta = kFusedCtaThreads / 32;
     const int V = tuning_.vector_width;
     auto resident = [&](int cluster, const FusedShape& f) {
         return mixed_ ? std::min(fused_max_clusters<float>(V, cluster, f), fused_max_clusters<double>(V, cluster, f))
                       : fused_max_clusters<double>(V, cluster, f);
     };
-    // The smallest cluster with a warp for every slice, up to 16 CTAs (8
+    // The smallest cluster with a worker for every slice, up to 16 CTAs (8
     // where the device cannot hold 16).
     int cluster = 1;
-    while (cluster < 16 && cluster * warps_per_cta < std::max(sh.slices_p, sh.slices_d)) cluster *= 2;
+    while (cluster < 16 && cluster * kFusedCtaWorkers < std::max(sh.slices_p, sh.slices_d)) cluster *= 2;
     if (cluster == 16 && resident(16, sh) <= 0) cluster = 8;
     if (resident(cluster, sh) <= 0) return;
-    // Staging: CTA rank r's warp q takes slice r * 16 + q of each side; its
-    // bytes at element size `elem`, with or without the lines' own iterates.
-    auto stage_bytes = [&](int own_p, int own_d, int elem) {
+    // Staging: CTA r takes slices r, r + C, ... of each side; the most bytes
+    // of a CTA.
+    auto stage_bytes = [&](int mode, int elem) {
         int64_t stage = 0;
         for (int b = 0; b < count_; ++b) {
             const InstanceInfo& inf = info_[static_cast<size_t>(b)];
@@ -940,39 +937,40 @@ void Engine::choose_fused() {
             const int ps1 = last(at_ctas_, inf.at_cta_end) - inf.at_slice_base;
             const int ds0 = first(a_ctas_, inf.a_cta_begin) - inf.a_slice_base;
             const int ds1 = last(a_ctas_, inf.a_cta_end) - inf.a_slice_base;
-            for (int r = 0; r < cluster; ++r) {
-                int64_t cta = 0;
-                for (int q = 0; q < warps_per_cta; ++q) {
-                    const int k = r * warps_per_cta + q;
-                    if (ps0 + k < ps1)
-                        cta += fused_slice_bytes(L.at.slices[static_cast<size_t>(ps0 + k)].steps,
-                                                 kFusedPrimalConsts + own_p, elem);
-                    if (ds0 + k < ds1)
-                        cta += fused_slice_bytes(L.a.slices[static_cast<size_t>(ds0 + k)].steps,
-                                                 kFusedDualConsts + own_d, elem);
-                }
-                stage = std::max(stage, cta);
-            }
+            std::vector<int64_t> cta(static_cast<size_t>(cluster), 0);
+            for (int s = ps0; s < ps1; ++s)
+                cta[static_cast<size_t>((s - ps0) % cluster)] += fused_slice_bytes(
+                    L.at.slices[static_cast<size_t>(s)].steps, kFusedPrimalConsts + fused_own_primal(mode), elem);
+            for (int s = ds0; s < ds1; ++s)
+                cta[static_cast<size_t>((s - ds0) % cluster)] += fused_slice_bytes(
+                    L.a.slices[static_cast<size_t>(s)].steps, kFusedDualConsts + fused_own_dual(mode), elem);
+            stage = std::max(stage, *std::max_element(cta.begin(), cta.end()));
         }
-        // Never zero when staged (the kernel tells the modes apart by it).
-        return static_cast<int32_t>(std::max<int64_t>(16, std::min<int64_t>(stage, INT32_MAX)));
+        return static_cast<int32_t>(std::min<int64_t>(stage, INT32_MAX));
     };
-    int32_t lines = 0;
-    for (int b = 0; b < count_; ++b)
-        lines = std::max(lines, info_[static_cast<size_t>(b)].m + info_[static_cast<size_t>(b)].n);
-    // Per working precision: copies of x and y if they fit, else the staged
-    // slices if they fit, else neither.
+    // A staged slice holds line numbers, lengths and indices in 16 bits.
+    bool narrow = true;
+    for (int b = 0; b < count_; ++b) {
+        const InstanceInfo& inf = info_[static_cast<size_t>(b)];
+        const MatrixLayout& L = layouts_[spec_.shared_matrix ? 0 : b];
+        narrow = narrow && inf.m < 65535 && inf.n < 65535;
+        for (const SideLayout* side : {&L.a, &L.at})
+            narrow = narrow && (side->line_len.empty() ||
+                                *std::max_element(side->line_len.begin(), side->line_len.end()) < 65536);
+    }
+    // Per working precision, the first layout that fits.
     auto best = [&](int elem, auto fits) {
         FusedShape out = sh;
         out.elem = elem;
-        if (cluster * warps_per_cta < std::max(sh.slices_p, sh.slices_d)) return out;
-        FusedShape copies = out;
-        copies.stage_bytes = stage_bytes(kFusedPrimalOwn, kFusedDualOwn, elem);
-        copies.lines = lines;
-        FusedShape staged = out;
-        staged.stage_bytes = stage_bytes(0, 0, elem);
-        if (fused_smem_bytes(copies) <= kFusedMaxSmemHost && fits(copies)) return copies;
-        if (fused_smem_bytes(staged) <= kFusedMaxSmemHost && fits(staged)) return staged;
+        if (kFusedLocal * cluster * kFusedCtaWorkers < std::max(sh.slices_p, sh.slices_d)) return out;
+        if (!narrow) return out;
+        for (const int mode : {kFusedCopies, kFusedHalf, kFusedStaged}) {
+            FusedShape f = out;
+            f.mode = mode;
+            f.stage_bytes = stage_bytes(mode, elem);
+            f.copied = mode == kFusedCopies ? cols_rows : mode == kFusedHalf ? rows : 0;
+            if (fused_smem_bytes(f) <= kFusedMaxSmemHost && fits(f)) return f;
+        }
         return out;
     };
     fused_shape64_ = best(static_cast<int>(sizeof(double)),

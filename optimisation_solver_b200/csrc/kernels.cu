@@ -457,742 +457,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_dual(Global g, Work<T> w, Devic
     }
 }
 
-// ---------------------------------------------------------------------------
-// Fused trials of small LPs: one thread-block cluster per instance runs the
-// trials of a check interval in one launch. Warp q of CTA rank r serves the
-// instance's slices r * kFusedWarps + q, stepping by the cluster's warp count;
-// per trial:
-//   primal half of every slice (k_primal's arithmetic, its warp sum per slice)
-//   cluster barrier
-//   dual half of every slice (k_dual's arithmetic)
-//   cluster barrier
-//   rank 0: each CTA-map entry's slice sums added in slice order (k_primal's
-//   and k_dual's block sums: one slice per warp, warps in order), then the
-//   entries' three sums in k_dual's fixed order and trial_control
-//   cluster barrier
-// so an instance's results are the two-kernel path's bit for bit, without a
-// launch, an arrival counter or a trip through the decision's dependent loads
-// per half. Vectors another CTA writes inside the launch (the iterates, the
-// partials, the control block) are read through L2 (ld.cg); the barrier's
-// release and acquire order them. Every CTA of a cluster reads the same
-// control block after the same barrier, so all of them leave the loop
-// together.
-// ---------------------------------------------------------------------------
-constexpr int kFusedGroups = 2;   // 512 threads: up to 128 registers each
-constexpr int kFusedThreads = kFusedGroups * kThreads;
-constexpr int kFusedWarps = kFusedThreads / 32;
-
-// Every thread of every CTA of the cluster; the warp is reconverged first
-// (the decision runs in one thread of rank 0's first warp just before).
-__device__ __forceinline__ void cluster_sync_all() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-
-// block_sum over one 256-thread group (its warps added in warp order, as
-// block_sum adds a CTA's); the result is valid in the group's thread 0.
-// Named barrier 1 + group; a second barrier frees `red` for the next call.
-// The lanes' values of one warp added by the butterfly of block_sum's first
-// stage (every lane gets the sum).
-template <int NQ>
-__device__ __forceinline__ void warp_sum(double (&v)[NQ]) {
-#pragma unroll
-    for (int q = 0; q < NQ; ++q)
-        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(kFull, v[q], o);
-}
-
-// The trial's snapshot of the control block, three 16-byte words.
-struct alignas(16) FusedCtl {
-    double mult_primal, mult_dual, frac;
-    int active, parity, pending, pad;
-};
-static_assert(sizeof(FusedCtl) == 48, "the snapshot travels as three 16-byte words");
-
-template <class T, int V>
-__device__ __forceinline__ double fused_primal(const Global& g, const Work<T>& w, const CtaWork& cw,
-                                               const InstanceInfo& inf, const FusedCtl& f, int lt) {
-    const int p = f.parity;
-    const T mult = static_cast<T>(f.mult_primal);
-    const bool pending = f.pending != 0;
-    const T frac = static_cast<T>(f.frac);
-    const T* y = w.Y[p] + inf.row_off;
-    const T* x = w.X[p] + inf.col_off;
-    T* xt = w.X[p ^ 1] + inf.col_off;
-    const T* cv = w.c + inf.col_off;
-    const T* lo = w.xl + inf.col_off;
-    const T* hi = w.xu + inf.col_off;
-    const T* tau = w.tau + inf.col_off;
-    const T* itau = w.itau + inf.col_off;
-    T* avg = w.avg_x + inf.col_off;
-    const T* vals = matrix_values<T>(g.at);
-    double moved = 0.0;
-    const int warp = lt >> 5, lane = lt & 31;
-    for (int s = cw.slice_begin + warp; s < cw.slice_end; s += kWarps) {
-        const SliceDesc sd = g.at.slices[s];
-        const LanePos lp = lane_pos(sd, lane);
-        const bool owner = lp.valid && lp.g == 0;
-        const int j = lp.line;
-        const int len = lp.valid ? g.at.line_len[inf.at_len_base + j] : 0;
-        T cj = T(0), prev = T(0), loj = T(0), hij = T(0), tj = T(0), itj = T(0), aj = T(0);
-        if (owner) {
-            cj = cv[j];
-            prev = __ldcg(x + j);
-            loj = lo[j];
-            hij = hi[j];
-            tj = tau[j];
-            itj = itau[j];
-            if (pending) aj = __ldcg(avg + j);
-        }
-        T sum[1] = {T(0)};
-        line_sums<V, 1>(inf.at_data_base + static_cast<int64_t>(sd.data_off) * 32, sd.steps, lp, lane, len,
-                        g.at.idx, vals, sum, [&](T (&a)[1], T v, int i) { a[0] += v * __ldcg(y + i); });
-        if (owner) {
-            const T gradient = cj + sum[0];
-            const T upd = smax(loj, smin(prev - mult * tj * gradient, hij));
-            xt[j] = upd;
-            const double d = static_cast<double>(upd - prev);
-            moved += d * d * static_cast<double>(itj);
-            if (pending) avg[j] = aj + frac * (prev - aj);
-        }
-    }
-    return moved;
-}
-
-template <class T, int V>
-__device__ __forceinline__ void fused_dual(const Global& g, const Work<T>& w, const CtaWork& cw,
-                                           const InstanceInfo& inf, const FusedCtl& f, int lt,
-                                           double (&red)[2]) {
-    const int p = f.parity;
-    const T dm = static_cast<T>(f.mult_dual);
-    const bool pending = f.pending != 0;
-    const T frac = static_cast<T>(f.frac);
-    const T* xt = w.X[p ^ 1] + inf.col_off;
-    const T* y = w.Y[p] + inf.row_off;
-    T* yt = w.Y[p ^ 1] + inf.row_off;
-    const T* ax = w.AX[p] + inf.row_off;
-    T* axt = w.AX[p ^ 1] + inf.row_off;
-    const T* lo = w.rl + inf.row_off;
-    const T* hi = w.ru + inf.row_off;
-    const T* sig = w.sigma + inf.row_off;
-    const T* isig = w.isigma + inf.row_off;
-    T* avg = w.avg_y + inf.row_off;
-    const T* vals = matrix_values<T>(g.a);
-    const int warp = lt >> 5, lane = lt & 31;
-    for (int s = cw.slice_begin + warp; s < cw.slice_end; s += kWarps) {
-        const SliceDesc sd = g.a.slices[s];
-        const LanePos lp = lane_pos(sd, lane);
-        const bool owner = lp.valid && lp.g == 0;
-        const int i = lp.line;
-        const int len = lp.valid ? g.a.line_len[inf.a_len_base + i] : 0;
-        T axi = T(0), sgi = T(0), prev = T(0), loi = T(0), hii = T(0), isi = T(0), ai = T(0);
-        if (owner) {
-            axi = __ldcg(ax + i);
-            sgi = sig[i];
-            prev = __ldcg(y + i);
-            loi = lo[i];
-            hii = hi[i];
-            isi = isig[i];
-            if (pending) ai = __ldcg(avg + i);
-        }
-        T sum[1] = {T(0)};
-        line_sums<V, 1, true>(inf.a_data_base + static_cast<int64_t>(sd.data_off) * 32, sd.steps, lp, lane, len,
-                              g.a.idx, vals, sum, [&](T (&a)[1], T v, int j) { a[0] += v * __ldcg(xt + j); });
-        if (owner) {
-            const T next = sum[0];
-            const T dact = next - axi;
-            const T ext = next + dact;
-            const T step = smax(dm * sgi, min_dual_step<T>());
-            const T v = prev + step * ext;
-            const T upd = smax(v - step * hii, T(0)) + smin(v - step * loi, T(0));
-            yt[i] = upd;
-            axt[i] = next;
-            const double d = static_cast<double>(upd - prev);
-            red[0] += d * d * static_cast<double>(isi);
-            red[1] += d * static_cast<double>(dact);
-            if (pending) avg[i] = ai + frac * (prev - ai);
-        }
-    }
-}
-
-// Distributed shared memory: the address of `local` in rank 0's shared
-// memory, and loads and stores there.
-__device__ __forceinline__ uint32_t rank0_addr(const void* local) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(local));
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(0));
-    return r;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-// The next trial's snapshot of an instance's control block.
-__device__ __forceinline__ void fused_snapshot(const InstanceCtl& c, FusedCtl& f, bool fp64) {
-    f.active = c.phase != kPhaseDone && c.stage == kStageTrial && (c.fp64_stage != 0) == fp64;
-    f.parity = c.parity;
-    f.pending = c.pending_avg;
-    f.mult_primal = c.trial_eta / c.trial_omega;
-    f.mult_dual = c.trial_eta * c.trial_omega;
-    f.frac = c.avg_frac;
-}
-
-static_assert(kFusedThreads == kFusedCtaThreads, "the engine sizes clusters by this CTA size");
-// Step factors a fused launch keeps in shared memory (trials past them read
-// the options' table).
-constexpr int kFusedFactors = 160;
-
-// Distributed shared memory of rank `r`: the address of `local` there, and
-// stores of the snapshot's fields.
-__device__ __forceinline__ uint32_t rank_addr(const void* local, uint32_t r) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(local));
-    uint32_t out;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(a), "r"(r));
-    return out;
-}
-__device__ __forceinline__ void st_cluster_i32(uint32_t addr, int v) {
-    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-
-// Lane r in [1, C) of rank 0's first warp copies the snapshot (written by lane
-// 0 before) into CTA r's `f`; the cluster barrier that follows publishes it.
-__device__ __forceinline__ void fused_publish(const FusedCtl& f, uint32_t C, int lane) {
-    __syncwarp();
-    if (lane >= 1 && static_cast<uint32_t>(lane) < C) {
-        const uint32_t a = rank_addr(&f, static_cast<uint32_t>(lane));
-        const int4* w = reinterpret_cast<const int4*>(&f);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const int4 v = w[q];
-            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a + 16u * q), "r"(v.x),
-                         "r"(v.y), "r"(v.z), "r"(v.w)
-                         : "memory");
-        }
-    }
-}
-
-// One warp's slice of one side, staged in shared memory for the launch: the
-// cluster barriers between the halves acquire at cluster scope, after which
-// the SM's L1 holds nothing of global memory, so the slice's entries and its
-// lines' constants would otherwise come from L2 in every trial.
-template <class T>
-struct FusedLane {
-    const int32_t* idx;   // [32 * steps], the layout of the slice data
-    const T* val;
-    const T* k;           // line constants [consts][32]
-    T* v;                 // the lines' own iterates [vecs][32] (launches with copies)
-    LanePos lp;
-    int steps, len;
-    bool has, owner;
-};
-
-// Carves the warp's region of one side: the slice's entries, its lines'
-// constants and, with copies, the lines' own iterates (`nvecs` vectors).
-template <class T>
-__device__ __forceinline__ void fused_stage(const Side& side, const T* vals, int64_t data_base, int len_base,
-                                            int s, bool has, unsigned char* dst, const T* const* consts,
-                                            int nconsts, const T* const* vecs, int nvecs, int lane,
-                                            FusedLane<T>& L) {
-    L.has = has;
-    L.owner = false;
-    L.steps = 0;
-    L.len = 0;
-    if (!has) return;
-    const SliceDesc sd = side.slices[s];
-    L.lp = lane_pos(sd, lane);
-    L.owner = L.lp.valid && L.lp.g == 0;
-    L.steps = sd.steps;
-    L.len = L.lp.valid ? side.line_len[len_base + L.lp.line] : 0;
-    int32_t* idx = reinterpret_cast<int32_t*>(dst);
-    T* val = reinterpret_cast<T*>(dst + 4 * 32 * sd.steps);
-    T* k = val + 32 * sd.steps;
-    const int64_t base = data_base + static_cast<int64_t>(sd.data_off) * 32;
-    for (int q = lane; q < 32 * sd.steps; q += 32) {
-        idx[q] = side.idx[base + q];
-        val[q] = vals[base + q];
-    }
-    for (int c = 0; c < nconsts; ++c) k[c * 32 + lane] = L.owner ? consts[c][L.lp.line] : T(0);
-    T* v = k + 32 * nconsts;
-    for (int c = 0; c < nvecs; ++c) v[c * 32 + lane] = L.owner ? vecs[c][L.lp.line] : T(0);
-    __syncwarp();
-    L.idx = idx;
-    L.val = val;
-    L.k = k;
-    L.v = v;
-}
-
-// line_sums over a staged slice: the same products added in the same order
-// (steps 0, 1, ... of the lane, then the lane group's butterfly), with eight
-// gathers in flight since the entries come from shared memory; `get(i)`
-// gathers element i of the other side's vector.
-template <int V, class T, class Get>
-__device__ __forceinline__ void staged_sums(const FusedLane<T>& L, int lane, Get get, T (&acc)[1]) {
-    constexpr int kAhead = 8;
-    for (int s0 = 0; s0 < L.steps; s0 += kAhead) {
-        T gv[kAhead], wv[kAhead];
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const int st = s0 + u;
-            gv[u] = T(0);
-            wv[u] = T(0);
-            if (st < L.steps && (st << L.lp.glog) + L.lp.g < L.len) {
-                const int q = (st / V) * (32 * V) + lane * V + st % V;
-                wv[u] = L.val[q];
-                gv[u] = get(L.idx[q]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const int st = s0 + u;
-            if (st < L.steps && (st << L.lp.glog) + L.lp.g < L.len) acc[0] += wv[u] * gv[u];
-        }
-    }
-    for (int o = (1 << L.lp.glog) >> 1; o > 0; o >>= 1) acc[0] += __shfl_xor_sync(kFull, acc[0], o);
-}
-
-// fused_primal over the warp's staged slice.
-template <class T, int V>
-__device__ __forceinline__ double fused_primal_staged(const Work<T>& w, const InstanceInfo& inf, const FusedCtl& f,
-                                                      const FusedLane<T>& L, int lane) {
-    const int p = f.parity;
-    const T mult = static_cast<T>(f.mult_primal);
-    const bool pending = f.pending != 0;
-    const T frac = static_cast<T>(f.frac);
-    const T* y = w.Y[p] + inf.row_off;
-    const T* x = w.X[p] + inf.col_off;
-    T* xt = w.X[p ^ 1] + inf.col_off;
-    T* avg = w.avg_x + inf.col_off;
-    const int j = L.lp.line;
-    T prev = T(0), aj = T(0);
-    if (L.owner) {
-        prev = __ldcg(x + j);
-        if (pending) aj = __ldcg(avg + j);
-    }
-    T sum[1] = {T(0)};
-    staged_sums<V>(L, lane, [&](int i) { return __ldcg(y + i); }, sum);
-    double moved = 0.0;
-    if (L.owner) {
-        const T cj = L.k[lane], loj = L.k[32 + lane], hij = L.k[64 + lane];
-        const T tj = L.k[96 + lane], itj = L.k[128 + lane];
-        const T gradient = cj + sum[0];
-        const T upd = smax(loj, smin(prev - mult * tj * gradient, hij));
-        xt[j] = upd;
-        const double d = static_cast<double>(upd - prev);
-        moved += d * d * static_cast<double>(itj);
-        if (pending) avg[j] = aj + frac * (prev - aj);
-    }
-    return moved;
-}
-
-// fused_dual over the warp's staged slice.
-template <class T, int V>
-__device__ __forceinline__ void fused_dual_staged(const Work<T>& w, const InstanceInfo& inf, const FusedCtl& f,
-                                                  const FusedLane<T>& L, int lane, double (&red)[2]) {
-    const int p = f.parity;
-    const T dm = static_cast<T>(f.mult_dual);
-    const bool pending = f.pending != 0;
-    const T frac = static_cast<T>(f.frac);
-    const T* xt = w.X[p ^ 1] + inf.col_off;
-    const T* y = w.Y[p] + inf.row_off;
-    T* yt = w.Y[p ^ 1] + inf.row_off;
-    const T* ax = w.AX[p] + inf.row_off;
-    T* axt = w.AX[p ^ 1] + inf.row_off;
-    T* avg = w.avg_y + inf.row_off;
-    const int i = L.lp.line;
-    T axi = T(0), prev = T(0), ai = T(0);
-    if (L.owner) {
-        axi = __ldcg(ax + i);
-        prev = __ldcg(y + i);
-        if (pending) ai = __ldcg(avg + i);
-    }
-    T sum[1] = {T(0)};
-    staged_sums<V>(L, lane, [&](int j) { return __ldcg(xt + j); }, sum);
-    if (L.owner) {
-        const T sgi = L.k[lane], isi = L.k[32 + lane], loi = L.k[64 + lane], hii = L.k[96 + lane];
-        const T next = sum[0];
-        const T dact = next - axi;
-        const T ext = next + dact;
-        const T step = smax(dm * sgi, min_dual_step<T>());
-        const T v = prev + step * ext;
-        const T upd = smax(v - step * hii, T(0)) + smin(v - step * loi, T(0));
-        yt[i] = upd;
-        axt[i] = next;
-        const double d = static_cast<double>(upd - prev);
-        red[0] += d * d * static_cast<double>(isi);
-        red[1] += d * static_cast<double>(dact);
-        if (pending) avg[i] = ai + frac * (prev - ai);
-    }
-}
-
-// Launches with copies: every CTA holds the instance's whole x and y (both
-// parities) in its shared memory, so the gathers are local; the owner lane of
-// a line writes its new value into every CTA's copy (the lanes of a slice own
-// consecutive lines, so each remote store is one contiguous run), and keeps
-// the line's average (and Ax) in its own region. No trial touches global
-// memory.
-template <class T>
-struct FusedCopies {
-    T* x[2];   // [n] each, this CTA's copy
-    T* y[2];   // [m] each
-};
-
-// The value v of element `e` of a copied vector, stored into all C copies.
-template <class T>
-__device__ __forceinline__ void store_copies(const T* elem, T v, uint32_t C);
-template <>
-__device__ __forceinline__ void store_copies<double>(const double* elem, double v, uint32_t C) {
-    for (uint32_t r = 0; r < C; ++r) st_cluster(rank_addr(elem, r), v);
-}
-template <>
-__device__ __forceinline__ void store_copies<float>(const float* elem, float v, uint32_t C) {
-    for (uint32_t r = 0; r < C; ++r)
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(rank_addr(elem, r)), "f"(v) : "memory");
-}
-
-// fused_primal with copies; own region: the line's average.
-template <class T, int V>
-__device__ __forceinline__ double fused_primal_copies(const FusedCtl& f, const FusedLane<T>& L,
-                                                      const FusedCopies<T>& cc, uint32_t C, int lane) {
-    const int p = f.parity;
-    const T mult = static_cast<T>(f.mult_primal);
-    const bool pending = f.pending != 0;
-    const T frac = static_cast<T>(f.frac);
-    const T* y = cc.y[p];
-    const int j = L.lp.line;
-    T prev = T(0), aj = T(0);
-    if (L.owner) {
-        prev = cc.x[p][j];
-        if (pending) aj = L.v[lane];
-    }
-    T sum[1] = {T(0)};
-    staged_sums<V>(L, lane, [&](int i) { return y[i]; }, sum);
-    double moved = 0.0;
-    if (L.owner) {
-        const T cj = L.k[lane], loj = L.k[32 + lane], hij = L.k[64 + lane];
-        const T tj = L.k[96 + lane], itj = L.k[128 + lane];
-        const T gradient = cj + sum[0];
-        const T upd = smax(loj, smin(prev - mult * tj * gradient, hij));
-        store_copies<T>(cc.x[p ^ 1] + j, upd, C);
-        const double d = static_cast<double>(upd - prev);
-        moved += d * d * static_cast<double>(itj);
-        if (pending) L.v[lane] = aj + frac * (prev - aj);
-    }
-    return moved;
-}
-
-// fused_dual with copies; own region: Ax of both parities, the average.
-template <class T, int V>
-__device__ __forceinline__ void fused_dual_copies(const FusedCtl& f, const FusedLane<T>& L,
-                                                  const FusedCopies<T>& cc, uint32_t C, int lane,
-                                                  double (&red)[2]) {
-    const int p = f.parity;
-    const T dm = static_cast<T>(f.mult_dual);
-    const bool pending = f.pending != 0;
-    const T frac = static_cast<T>(f.frac);
-    const T* xt = cc.x[p ^ 1];
-    const int i = L.lp.line;
-    T axi = T(0), prev = T(0), ai = T(0);
-    if (L.owner) {
-        axi = L.v[p * 32 + lane];
-        prev = cc.y[p][i];
-        if (pending) ai = L.v[64 + lane];
-    }
-    T sum[1] = {T(0)};
-    staged_sums<V>(L, lane, [&](int jj) { return xt[jj]; }, sum);
-    if (L.owner) {
-        const T sgi = L.k[lane], isi = L.k[32 + lane], loi = L.k[64 + lane], hii = L.k[96 + lane];
-        const T next = sum[0];
-        const T dact = next - axi;
-        const T ext = next + dact;
-        const T step = smax(dm * sgi, min_dual_step<T>());
-        const T v = prev + step * ext;
-        const T upd = smax(v - step * hii, T(0)) + smin(v - step * loi, T(0));
-        store_copies<T>(cc.y[p ^ 1] + i, upd, C);
-        L.v[(p ^ 1) * 32 + lane] = next;
-        const double d = static_cast<double>(upd - prev);
-        red[0] += d * d * static_cast<double>(isi);
-        red[1] += d * static_cast<double>(dact);
-        if (pending) L.v[64 + lane] = ai + frac * (prev - ai);
-    }
-}
-
-// One thread per CTA-map entry of rank 0 replaces the entry's slice sums
-// (`nq` values per slice) by their in-order total, stored at the entry's
-// first slice. Table word: first slice << 4 | slice count.
-__device__ __forceinline__ void fused_entry_totals(const int32_t* tab, int entries, double* part, int nq) {
-    for (int e = static_cast<int>(threadIdx.x); e < entries; e += kFusedThreads) {
-        const int first = tab[e] >> 4, cnt = tab[e] & 15;
-        if (cnt == 0) continue;
-        for (int q = 0; q < nq; ++q) {
-            double t = 0.0;
-            for (int k = 0; k < cnt; ++k) t += part[(first + k) * nq + q];
-            part[first * nq + q] = t;
-        }
-    }
-}
-
-__device__ __forceinline__ double fused_entry(const int32_t* tab, int e, const double* part, int nq, int q) {
-    return (tab[e] & 15) ? part[(tab[e] >> 4) * nq + q] : 0.0;
-}
-
-template <class T, int V>
-__global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w, DeviceOptions o,
-                                                           int max_trials, FusedShape fs) {
-    // Rank 0 keeps the instance's control block in its shared memory for the
-    // whole launch (the decision's reads and writes stay on chip), writes
-    // each trial's snapshot into every CTA's `f`, and receives every slice's
-    // warp sums in `part_p` / `part_d` through distributed shared memory. The
-    // block goes back to global memory when the launch ends.
-    __shared__ DeviceOptions so;
-    __shared__ FusedCtl f;
-    __shared__ alignas(16) InstanceCtl sctl;
-    // Rank 0: step_pow entries of iteration indices fac0 .. fac0 + nfac - 1.
-    __shared__ double sfac[2 * kFusedFactors];
-    __shared__ int64_t fac0;
-    __shared__ int nfac;
-    extern __shared__ __align__(16) unsigned char fused_smem[];
-    double* const part_p = reinterpret_cast<double*>(fused_smem);
-    double* const part_d = part_p + fs.slices_p;
-    int32_t* const tab_p = reinterpret_cast<int32_t*>(part_d + 2 * fs.slices_d);
-    int32_t* const tab_d = tab_p + fs.entries_p;
-    unsigned char* const stage = fused_smem + fused_stage_offset(fs);
-    T* const copies = reinterpret_cast<T*>(fused_smem + fused_copies_offset(fs));
-    const uint32_t C = cluster_size(), rank = cluster_rank();
-    const int b = static_cast<int>(blockIdx.x / C);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    InstanceCtl* cp = g.ctl + b;
-    const InstanceInfo inf = g.info[b];
-    // The instance's slices are contiguous in its CTA map (append_cta_map).
-    const int ps0 = g.at.ctas[inf.at_cta_begin].slice_begin, ps1 = g.at.ctas[inf.at_cta_end - 1].slice_end;
-    const int ds0 = g.a.ctas[inf.a_cta_begin].slice_begin, ds1 = g.a.ctas[inf.a_cta_end - 1].slice_end;
-    const int ne_p = inf.at_cta_end - inf.at_cta_begin, ne_d = inf.a_cta_end - inf.a_cta_begin;
-    // One warp per slice: slice s goes to warp s mod (cluster warps).
-    const int stride = static_cast<int>(C) * kFusedWarps;
-    const int slot = static_cast<int>(rank) * kFusedWarps + warp;
-    constexpr bool kFp64 = sizeof(T) == 8;
-    const T* vals_p = matrix_values<T>(g.at);
-    const T* vals_d = matrix_values<T>(g.a);
-    if (threadIdx.x == 0) so = o;
-    if (rank == 0) {
-        static_assert(sizeof(InstanceCtl) % 16 == 0, "the control block copies as 16-byte words");
-        if (threadIdx.x < sizeof(InstanceCtl) / 16)
-            reinterpret_cast<int4*>(&sctl)[threadIdx.x] = reinterpret_cast<const int4*>(cp)[threadIdx.x];
-        for (int e = threadIdx.x; e < ne_p; e += kFusedThreads) {
-            const CtaWork cw = g.at.ctas[inf.at_cta_begin + e];
-            tab_p[e] = ((cw.slice_begin - ps0) << 4) | (cw.slice_end - cw.slice_begin);
-        }
-        for (int e = threadIdx.x; e < ne_d; e += kFusedThreads) {
-            const CtaWork cw = g.a.ctas[inf.a_cta_begin + e];
-            tab_d[e] = ((cw.slice_begin - ds0) << 4) | (cw.slice_end - cw.slice_begin);
-        }
-        // The linesearch's step factors of the launch's iteration indices
-        // (one phase per launch: a phase ends at a check, which ends it).
-        {
-            const InstanceCtl& c0 = *cp;
-            const int64_t k0 = c0.phase == kPhasePolish ? c0.polish_iteration : c0.iteration;
-            const int64_t avail = k0 >= 0 && k0 < o.step_pow_entries ? o.step_pow_entries - k0 : 0;
-            const int n = static_cast<int>(avail < kFusedFactors ? avail : kFusedFactors);
-            for (int q = threadIdx.x; q < 2 * n; q += kFusedThreads) sfac[q] = o.step_pow[2 * k0 + q];
-            if (threadIdx.x == 0) {
-                fac0 = k0;
-                nfac = n;
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) fused_snapshot(sctl, f, kFp64);
-    }
-    // Staged launches give every warp at most one slice per side; with
-    // copies, the x and y of both parities are in every CTA.
-    const bool staged = fs.stage_bytes > 0 && fs.elem == static_cast<int>(sizeof(T));
-    const bool with_copies = staged && fs.lines > 0;
-    FusedLane<T> LP{}, LD{};
-    FusedCopies<T> cc{};
-    T* const xg[2] = {w.X[0] + inf.col_off, w.X[1] + inf.col_off};
-    T* const yg[2] = {w.Y[0] + inf.row_off, w.Y[1] + inf.row_off};
-    // The lines' own iterates with copies: primal the average; dual Ax of
-    // both parities, the average.
-    const T* const own_p[1] = {w.avg_x + inf.col_off};
-    const T* const own_d[3] = {w.AX[0] + inf.row_off, w.AX[1] + inf.row_off, w.avg_y + inf.row_off};
-    const int words_p = kFusedPrimalConsts + (with_copies ? kFusedPrimalOwn : 0);
-    const int words_d = kFusedDualConsts + (with_copies ? kFusedDualOwn : 0);
-    if (with_copies) {
-        cc.x[0] = copies;
-        cc.x[1] = copies + inf.n;
-        cc.y[0] = copies + 2 * inf.n;
-        cc.y[1] = copies + 2 * inf.n + inf.m;
-        for (int q = threadIdx.x; q < inf.n; q += kFusedThreads) {
-            cc.x[0][q] = xg[0][q];
-            cc.x[1][q] = xg[1][q];
-        }
-        for (int q = threadIdx.x; q < inf.m; q += kFusedThreads) {
-            cc.y[0][q] = yg[0][q];
-            cc.y[1][q] = yg[1][q];
-        }
-    }
-    if (staged) {
-        // The warps' shares of the stage, in warp order (lane q of every
-        // warp computes warp q's bytes).
-        const int sp = ps0 + static_cast<int>(rank) * kFusedWarps + lane;
-        const int sd = ds0 + static_cast<int>(rank) * kFusedWarps + lane;
-        int need = 0;
-        if (lane < kFusedWarps) {
-            if (sp < ps1) need += fused_slice_bytes(g.at.slices[sp].steps, words_p, sizeof(T));
-            if (sd < ds1) need += fused_slice_bytes(g.a.slices[sd].steps, words_d, sizeof(T));
-        }
-        int incl = need;
-        for (int d = 1; d < 32; d <<= 1) {
-            const int t = __shfl_up_sync(kFull, incl, d);
-            if (lane >= d) incl += t;
-        }
-        const int off = __shfl_sync(kFull, incl - need, warp);
-        const int s_p = ps0 + slot, s_d = ds0 + slot;
-        const T* const cp_consts[kFusedPrimalConsts] = {w.c + inf.col_off, w.xl + inf.col_off, w.xu + inf.col_off,
-                                                        w.tau + inf.col_off, w.itau + inf.col_off};
-        const T* const cd_consts[kFusedDualConsts] = {w.sigma + inf.row_off, w.isigma + inf.row_off,
-                                                      w.rl + inf.row_off, w.ru + inf.row_off};
-        fused_stage<T>(g.at, vals_p, inf.at_data_base, inf.at_len_base, s_p, s_p < ps1, stage + off, cp_consts,
-                       kFusedPrimalConsts, own_p, with_copies ? kFusedPrimalOwn : 0, lane, LP);
-        const int off_d = off + (s_p < ps1 ? fused_slice_bytes(LP.steps, words_p, sizeof(T)) : 0);
-        fused_stage<T>(g.a, vals_d, inf.a_data_base, inf.a_len_base, s_d, s_d < ds1, stage + off_d, cd_consts,
-                       kFusedDualConsts, own_d, with_copies ? kFusedDualOwn : 0, lane, LD);
-    }
-    const uint32_t pp_addr = rank0_addr(part_p);
-    const uint32_t pd_addr = rank0_addr(part_d);
-    // Remote shared memory is written only once every CTA of the cluster
-    // runs: the first snapshot goes out after a barrier.
-    cluster_sync_all();
-    if (rank == 0 && threadIdx.x < 32) fused_publish(f, C, lane);
-    cluster_sync_all();
-    for (int t = 0; t < max_trials; ++t) {
-        if (!f.active) break;
-        if (with_copies) {
-            if (LP.has) {
-                double v[1] = {fused_primal_copies<T, V>(f, LP, cc, C, lane)};
-                warp_sum<1>(v);
-                if (lane == 0) st_cluster(pp_addr + 8u * static_cast<uint32_t>(slot), v[0]);
-            }
-        } else if (staged) {
-            if (LP.has) {
-                double v[1] = {fused_primal_staged<T, V>(w, inf, f, LP, lane)};
-                warp_sum<1>(v);
-                if (lane == 0) st_cluster(pp_addr + 8u * static_cast<uint32_t>(ps0 + slot - ps0), v[0]);
-            }
-        } else {
-            for (int s = ps0 + slot; s < ps1; s += stride) {
-                const CtaWork one{b, s, s + 1, 0};
-                double v[1] = {fused_primal<T, V>(g, w, one, inf, f, lane)};
-                warp_sum<1>(v);
-                if (lane == 0) st_cluster(pp_addr + 8u * static_cast<uint32_t>(s - ps0), v[0]);
-            }
-        }
-        cluster_sync_all();
-        if (with_copies) {
-            if (LD.has) {
-                double r2[2] = {0.0, 0.0};
-                fused_dual_copies<T, V>(f, LD, cc, C, lane, r2);
-                warp_sum<2>(r2);
-                if (lane == 0) {
-                    const uint32_t q = 16u * static_cast<uint32_t>(slot);
-                    st_cluster(pd_addr + q, r2[0]);
-                    st_cluster(pd_addr + q + 8u, r2[1]);
-                }
-            }
-        } else if (staged) {
-            if (LD.has) {
-                double r2[2] = {0.0, 0.0};
-                fused_dual_staged<T, V>(w, inf, f, LD, lane, r2);
-                warp_sum<2>(r2);
-                if (lane == 0) {
-                    const uint32_t q = 16u * static_cast<uint32_t>(slot);
-                    st_cluster(pd_addr + q, r2[0]);
-                    st_cluster(pd_addr + q + 8u, r2[1]);
-                }
-            }
-        } else {
-            for (int s = ds0 + slot; s < ds1; s += stride) {
-                const CtaWork one{b, s, s + 1, 0};
-                double r2[2] = {0.0, 0.0};
-                fused_dual<T, V>(g, w, one, inf, f, lane, r2);
-                warp_sum<2>(r2);
-                if (lane == 0) {
-                    const uint32_t q = 16u * static_cast<uint32_t>(s - ds0);
-                    st_cluster(pd_addr + q, r2[0]);
-                    st_cluster(pd_addr + q + 8u, r2[1]);
-                }
-            }
-        }
-        cluster_sync_all();
-        if (rank == 0) {
-            if (fs.multi) {
-                // (With one slice per entry an entry's total, 0 + its slice's
-                // sum, is that sum: a sum of lane values that start at +0 is
-                // never -0.)
-                fused_entry_totals(tab_p, ne_p, part_p, 1);
-                fused_entry_totals(tab_d, ne_d, part_d, 2);
-                __syncthreads();
-            }
-            if (threadIdx.x < 32) {
-                // k_dual's fixed-order sums over the entries' totals
-                // (warp_range_sums3: entries lane, lane + 32, ... in order,
-                // then the butterfly).
-                double sums[3] = {0.0, 0.0, 0.0};
-                for (int e = lane; e < ne_p; e += 32) sums[0] += fused_entry(tab_p, e, part_p, 1, 0);
-                for (int e = lane; e < ne_d; e += 32) {
-                    sums[1] += fused_entry(tab_d, e, part_d, 2, 0);
-                    sums[2] += fused_entry(tab_d, e, part_d, 2, 1);
-                }
-                warp_sum<3>(sums);
-                if (threadIdx.x == 0) {
-                    const int64_t k = sctl.phase == kPhasePolish ? sctl.polish_iteration : sctl.iteration;
-                    const double* fk = k >= fac0 && k - fac0 < nfac ? sfac + 2 * (k - fac0) : nullptr;
-                    trial_control(sctl, so, sums[0], sums[1], sums[2], inf.n, fk);
-                    fused_snapshot(sctl, f, kFp64);
-                }
-                fused_publish(f, C, lane);
-            }
-        }
-        cluster_sync_all();
-    }
-    // Every CTA left the loop at the same trial (the same snapshot after the
-    // same barrier); the barrier keeps every CTA's shared memory alive until
-    // the last remote store into it has landed.
-    cluster_sync_all();
-    if (with_copies) {
-        // Every copy is the same: rank 0 writes x and y back, the owner lanes
-        // their lines' own iterates.
-        if (rank == 0) {
-            for (int q = threadIdx.x; q < inf.n; q += kFusedThreads) {
-                xg[0][q] = cc.x[0][q];
-                xg[1][q] = cc.x[1][q];
-            }
-            for (int q = threadIdx.x; q < inf.m; q += kFusedThreads) {
-                yg[0][q] = cc.y[0][q];
-                yg[1][q] = cc.y[1][q];
-            }
-        }
-        if (LP.has && LP.owner) w.avg_x[inf.col_off + LP.lp.line] = LP.v[lane];
-        if (LD.has && LD.owner) {
-            const int i = inf.row_off + LD.lp.line;
-            w.AX[0][i] = LD.v[lane];
-            w.AX[1][i] = LD.v[32 + lane];
-            w.avg_y[i] = LD.v[64 + lane];
-        }
-    }
-    if (rank == 0) {
-        if (threadIdx.x < sizeof(InstanceCtl) / 16)
-            reinterpret_cast<int4*>(cp)[threadIdx.x] = reinterpret_cast<const int4*>(&sctl)[threadIdx.x];
-    }
-}
+// Fused trials of small LPs (k_fused).
+#include "fused.cuh"
 
 // ---------------------------------------------------------------------------
 // Check, elementwise part (termination.cpp rowPass/columnPass terms without a
@@ -2305,59 +1571,48 @@ void launch_primal(const Global& g, const Work<T>& w, const DeviceOptions&, int 
 }
 
 namespace {
-template <class T, int V>
-cudaError_t fused_v(const Global& g, const Work<T>& w, const DeviceOptions& o, int count, int cluster,
-                    int max_trials, const FusedShape& shape, cudaStream_t s) {
+// The fused kernel of a shape: staged ones by layout and by whether a worker
+// has one slice a side (the code of one slice is a quarter as long, and a
+// trial is as fast as its instructions come in) or up to kFusedLocal.
+template <class T, int NL>
+auto fused_kernel(int mode) {
+    switch (mode) {
+        case kFusedCopies: return k_fused<T, kFusedCopies, NL>;
+        case kFusedHalf: return k_fused<T, kFusedHalf, NL>;
+        default: return k_fused<T, kFusedStaged, NL>;
+    }
+}
+
+template <class T>
+auto fused_kernel(int vw, int cluster, const FusedShape& f) {
+    if (f.mode == kFusedGlobal)
+        return vw == 4 ? k_fused_global<T, 4> : vw == 2 ? k_fused_global<T, 2> : k_fused_global<T, 1>;
+    return std::max(f.slices_p, f.slices_d) <= cluster * kFusedCtaWorkers ? fused_kernel<T, 1>(f.mode)
+                                                                          : fused_kernel<T, kFusedLocal>(f.mode);
+}
+
+// The launch configuration of `count` clusters; false where the device
+// refuses it.
+template <class K>
+bool fused_config(K kernel, int count, int cluster, const FusedShape& shape, cudaLaunchConfig_t& cfg,
+                  cudaLaunchAttribute& attr) {
     const size_t smem = fused_smem_bytes(shape);
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_fused<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
+    cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(count * cluster));
     cfg.blockDim = dim3(kFusedThreads);
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
     cfg.numAttrs = 1;
     // Clusters of 16 CTAs are beyond the portable size of 8.
-    cudaFuncSetAttribute(k_fused<T, V>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return cudaLaunchKernelEx(&cfg, k_fused<T, V>, g, w, o, max_trials, shape);
-}
-
-template <class T, int V>
-int fused_clusters_v(int cluster, size_t smem) {
-    if (cudaFuncSetAttribute(k_fused<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(cluster));
-    cfg.blockDim = dim3(kFusedThreads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cluster > 8 &&
-        cudaFuncSetAttribute(k_fused<T, V>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_fused<T, V>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return n;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    return false;
 }
 }  // namespace
 
@@ -2365,21 +1620,26 @@ template <class T>
 cudaError_t launch_fused(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw, int count,
                          int cluster, int max_trials, const FusedShape& shape, cudaStream_t s) {
     if (count <= 0) return cudaSuccess;
-    switch (vw) {
-        case 4: return fused_v<T, 4>(g, w, o, count, cluster, max_trials, shape, s);
-        case 2: return fused_v<T, 2>(g, w, o, count, cluster, max_trials, shape, s);
-        default: return fused_v<T, 1>(g, w, o, count, cluster, max_trials, shape, s);
-    }
+    auto* kernel = fused_kernel<T>(vw, cluster, shape);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    if (!fused_config(kernel, count, cluster, shape, cfg, attr)) return cudaErrorInvalidConfiguration;
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, kernel, g, w, o, vw == 4 ? 2 : vw == 2 ? 1 : 0, max_trials, shape);
 }
 
 template <class T>
 int fused_max_clusters(int vw, int cluster, const FusedShape& shape) {
-    const size_t smem = fused_smem_bytes(shape);
-    switch (vw) {
-        case 4: return fused_clusters_v<T, 4>(cluster, smem);
-        case 2: return fused_clusters_v<T, 2>(cluster, smem);
-        default: return fused_clusters_v<T, 1>(cluster, smem);
+    auto* kernel = fused_kernel<T>(vw, cluster, shape);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    if (!fused_config(kernel, 1, cluster, shape, cfg, attr)) return 0;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
+    return n;
 }
 
 template <class T>

@@ -107,51 +107,56 @@ void launch_primal(const Global& g, const Work<T>& w, const DeviceOptions& o, in
 template <class T>
 void launch_dual(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw,
                  cudaStream_t s);
+// Where a fused launch keeps its vectors (fused.cuh).
+enum : int32_t { kFusedGlobal = 0, kFusedStaged = 1, kFusedHalf = 2, kFusedCopies = 3 };
 // The shape of a fused launch's shared memory, over its instances.
 struct FusedShape {
+    int32_t mode;                   // kFused*
     int32_t slices_p, slices_d;     // most slices of an instance per side
     int32_t entries_p, entries_d;   // most CTA-map entries of an instance per side
-    int32_t stage_bytes;            // most bytes of a CTA's staged slices (0: nothing staged)
-    int32_t lines;                  // staged with copies: most rows + columns of an instance (else 0)
-    int32_t multi;                  // some CTA-map entry has other than one slice
+    int32_t stage_bytes;            // most bytes of a CTA's staged slices
+    int32_t copied;                 // most elements of an instance's copied vectors
     int32_t elem;                   // bytes of the launch's working precision
 };
-// Dynamic shared memory of a fused CTA: one warp sum per primal slice, two
-// per dual slice, one word per CTA-map entry; then, with copies, x and y of
-// both parities; then the staged slices.
+// Dynamic shared memory of a fused CTA: two sets of a warp sum per primal
+// slice, two sums per dual slice, one word per CTA-map entry; then the copied
+// vectors; then the staged slices.
 __host__ __device__ inline size_t fused_copies_offset(const FusedShape& f) {
-    const size_t b = sizeof(double) * (static_cast<size_t>(f.slices_p) + 2 * static_cast<size_t>(f.slices_d)) +
+    const size_t b = sizeof(double) * (2 * static_cast<size_t>(f.slices_p) + 2 * static_cast<size_t>(f.slices_d)) +
                      sizeof(int32_t) * (static_cast<size_t>(f.entries_p) + static_cast<size_t>(f.entries_d));
     return (b + 15) & ~static_cast<size_t>(15);
 }
 __host__ __device__ inline size_t fused_stage_offset(const FusedShape& f) {
-    return fused_copies_offset(f) + 2 * static_cast<size_t>(f.elem) * static_cast<size_t>(f.lines);
+    const size_t b = fused_copies_offset(f) + static_cast<size_t>(f.elem) * static_cast<size_t>(f.copied);
+    return (b + 15) & ~static_cast<size_t>(15);
 }
 __host__ __device__ inline size_t fused_smem_bytes(const FusedShape& f) {
     return fused_stage_offset(f) + static_cast<size_t>(f.stage_bytes);
 }
-// A staged slice in shared memory: the index and value of each of its 32 x
-// `steps` entries, then `consts` line constants per lane (element size
-// `elem`).
+// A staged slice in shared memory: a head word per lane, the index (16 bits)
+// and value of each of its 32 x `steps` entries, then the lines' constants
+// and own vectors, `words` per lane (element size `elem`).
+constexpr int kFusedHeadBytes = 128;
 constexpr int kFusedPrimalConsts = 5;   // objective, lower, upper, tau, 1/tau
 constexpr int kFusedDualConsts = 4;     // sigma, 1/sigma, lower, upper
-// With copies, the lines' own iterates follow the constants.
-constexpr int kFusedPrimalOwn = 1;      // the average
-constexpr int kFusedDualOwn = 3;        // Ax of both parities, the average
-__host__ __device__ constexpr int fused_slice_bytes(int steps, int consts, int elem) {
-    return 32 * steps * (4 + elem) + 32 * consts * elem;
+// Own vectors: the average and x of both parities; Ax of both parities, the
+// average and, where y is not copied, y of both.
+__host__ __device__ constexpr int fused_own_primal(int) { return 3; }
+__host__ __device__ constexpr int fused_own_dual(int mode) { return mode == kFusedStaged ? 5 : 3; }
+__host__ __device__ constexpr int fused_slice_bytes(int steps, int words, int elem) {
+    return kFusedHeadBytes + 32 * steps * (2 + elem) + 32 * words * elem;
 }
+constexpr int kFusedCtaWorkers = 16;    // worker warps of a CTA (and one that decides)
+constexpr int kFusedLocal = 4;          // staged slices of a worker per side at most
 // The trials of a check interval of `count` small instances in one launch:
-// one cluster of `cluster` CTAs (512 threads each) per instance, at most
-// `max_trials` trials each, stopping at a check or the end (kernels.cu,
-// k_fused). Same results as launch_primal + launch_dual per trial.
+// one cluster of `cluster` CTAs per instance, at most
+// `max_trials` trials each, stopping at a check or the end (fused.cuh). Same results as launch_primal + launch_dual per trial.
 template <class T>
 cudaError_t launch_fused(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw, int count,
                          int cluster, int max_trials, const FusedShape& shape, cudaStream_t s);
 // Clusters of that shape resident at once (0: the launch is not possible).
 template <class T>
 int fused_max_clusters(int vw, int cluster, const FusedShape& shape);
-constexpr int kFusedCtaThreads = 512;
 // Largest dynamic shared memory the engine gives a fused CTA (its static
 // shared memory, the control block and the options, fit beside it).
 constexpr size_t kFusedMaxSmemHost = 220 * 1024;
