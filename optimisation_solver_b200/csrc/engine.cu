@@ -123,20 +123,43 @@ void Engine::mark(const char* phase) {
 }
 
 namespace {
-constexpr size_t kPinnedChunk = size_t(64) << 20;   // bytes per staging buffer
+constexpr size_t kPinnedMin = size_t(4) << 20;      // bytes per staging buffer
+constexpr size_t kPinnedMax = size_t(64) << 20;
 constexpr size_t kPinnedDirect = size_t(4) << 20;   // smaller uploads go as they are
-constexpr size_t kCopyJob = size_t(2) << 20;        // host memcpy piece per thread
+
+// Host memcpy piece per thread: about 16 of a chunk, so that a small chunk has
+// as many threads copying as the memory needs.
+size_t copy_job(size_t chunk) {
+    return std::min(std::max(chunk / 16, size_t(256) << 10), size_t(2) << 20);
+}
 }  // namespace
 
-bool Engine::ensure_pinned() {
+// Bytes per staging buffer for a copy of `total` bytes. Pinning costs about
+// 0.7 ms a MiB and a chunk about 0.3 ms (its threads, its wait), so of T MiB in
+// chunks of c the overhead 1.4 c + 0.3 T / c is least at c = sqrt(0.2 T): 8 MiB
+// for 300 MiB, the full 64 MiB from 20 GiB. Two buffers of 64 MiB for any copy
+// cost 73 to 110 ms, half of a solve of 48 LPs of 200 to 10000 rows. An engine
+// whose later copies are much larger takes larger buffers then.
+bool Engine::ensure_pinned(size_t total) {
+    const double mib = static_cast<double>(total) / (1 << 20);
+    const size_t want = static_cast<size_t>(std::sqrt(0.2 * mib) * 4.0) << 18;   // in steps of 256 KiB
+    const size_t chunk = std::min(std::max(want, kPinnedMin), kPinnedMax);
+    if (pinned_chunk_ != 0 && chunk <= 2 * pinned_chunk_) return true;
     for (int b = 0; b < 2; ++b) {
-        if (pinned_[b] == nullptr &&
-            !check(cudaHostAlloc(reinterpret_cast<void**>(&pinned_[b]), kPinnedChunk, cudaHostAllocDefault), "cudaHostAlloc"))
+        if (pinned_done_[b] == nullptr) {
+            if (!check(cudaEventCreateWithFlags(&pinned_done_[b], cudaEventDisableTiming), "cudaEventCreate")) return false;
+        } else if (!check(cudaEventSynchronize(pinned_done_[b]), "staging")) {
             return false;
-        if (pinned_done_[b] == nullptr &&
-            !check(cudaEventCreateWithFlags(&pinned_done_[b], cudaEventDisableTiming), "cudaEventCreate"))
+        }
+    }
+    pinned_chunk_ = 0;
+    for (int b = 0; b < 2; ++b) {
+        if (pinned_[b] != nullptr) cudaFreeHost(pinned_[b]);
+        pinned_[b] = nullptr;
+        if (!check(cudaHostAlloc(reinterpret_cast<void**>(&pinned_[b]), chunk, cudaHostAllocDefault), "cudaHostAlloc"))
             return false;
     }
+    pinned_chunk_ = chunk;
     return true;
 }
 
@@ -147,10 +170,10 @@ bool Engine::download(void* dst, const void* src, size_t bytes) {
     if (bytes < kPinnedDirect)
         return check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_), "download") &&
                check(cudaStreamSynchronize(stream_), "download");
-    if (!ensure_pinned()) return false;
-    const size_t chunks = (bytes + kPinnedChunk - 1) / kPinnedChunk;
+    if (!ensure_pinned(bytes)) return false;
+    const size_t chunks = (bytes + pinned_chunk_ - 1) / pinned_chunk_;
     auto enqueue = [&](size_t c) {
-        const size_t off = c * kPinnedChunk, n = std::min(kPinnedChunk, bytes - off);
+        const size_t off = c * pinned_chunk_, n = std::min(pinned_chunk_, bytes - off);
         return check(cudaMemcpyAsync(pinned_[c & 1], static_cast<const char*>(src) + off, n, cudaMemcpyDeviceToHost, stream_), "download") &&
                check(cudaEventRecord(pinned_done_[c & 1], stream_), "download");
     };
@@ -158,13 +181,14 @@ bool Engine::download(void* dst, const void* src, size_t bytes) {
     for (size_t c = 0; c < chunks; ++c) {
         if (c + 1 < chunks && !enqueue(c + 1)) return false;
         if (!check(cudaEventSynchronize(pinned_done_[c & 1]), "download")) return false;
-        const size_t off = c * kPinnedChunk, n = std::min(kPinnedChunk, bytes - off);
-        const int jobs = static_cast<int>((n + kCopyJob - 1) / kCopyJob);
+        const size_t off = c * pinned_chunk_, n = std::min(pinned_chunk_, bytes - off);
+        const size_t cut = copy_job(n);
+        const int jobs = static_cast<int>((n + cut - 1) / cut);
         const char* from = pinned_[c & 1];
         char* to = static_cast<char*>(dst) + off;
         parallel_for(jobs, [&](int j) {
-            const size_t a = static_cast<size_t>(j) * kCopyJob;
-            std::memcpy(to + a, from + a, std::min(kCopyJob, n - a));
+            const size_t a = static_cast<size_t>(j) * cut;
+            std::memcpy(to + a, from + a, std::min(cut, n - a));
         });
     }
     return true;
@@ -173,7 +197,7 @@ bool Engine::download(void* dst, const void* src, size_t bytes) {
 // A copy from pageable memory is staged by the driver through its own small
 // pinned buffers, one thread, and returns only when it is done: for the
 // gigabytes of a large batch's matrices that runs at a fraction of the host
-// link. Large uploads here go through two 64 MiB pinned buffers instead: all
+// link. Large uploads here go through two pinned buffers instead: all
 // host threads fill one while the other's DMA is in flight.
 bool Engine::upload(void* dst, const std::vector<HostPiece>& pieces) {
     size_t total = 0;
@@ -188,23 +212,24 @@ bool Engine::upload(void* dst, const std::vector<HostPiece>& pieces) {
         }
         return true;
     }
-    if (!ensure_pinned()) return false;
+    if (!ensure_pinned(total)) return false;
     struct Job {
         size_t at;          // offset in the staging buffer
         const char* src;
         size_t bytes;
     };
     std::vector<Job> jobs;
+    const size_t cut = copy_job(std::min(total, pinned_chunk_));
     size_t piece = 0, in_piece = 0;   // read position
     for (int chunk = 0; piece < pieces.size(); ++chunk) {
         const int b = chunk & 1;
-        // Jobs of this chunk: up to kPinnedChunk bytes of the pieces, cut
-        // into at most kCopyJob bytes each.
+        // Jobs of this chunk: up to pinned_chunk_ bytes of the pieces, cut
+        // into at most `cut` bytes each.
         jobs.clear();
         size_t fill = 0;
-        while (fill < kPinnedChunk && piece < pieces.size()) {
+        while (fill < pinned_chunk_ && piece < pieces.size()) {
             const HostPiece& q = pieces[piece];
-            const size_t n = std::min({q.bytes - in_piece, kPinnedChunk - fill, kCopyJob});
+            const size_t n = std::min({q.bytes - in_piece, pinned_chunk_ - fill, cut});
             if (n > 0) jobs.push_back({fill, static_cast<const char*>(q.src) + in_piece, n});
             fill += n;
             in_piece += n;
@@ -306,9 +331,8 @@ bool Engine::prepare(const SolveSpec& spec) {
 
     // --- device and tuning ------------------------------------------------
     if (!check(cudaSetDevice(device_), "cudaSetDevice")) return false;
-    cudaDeviceProp prop;
-    if (!check(cudaGetDeviceProperties(&prop, device_), "cudaGetDeviceProperties")) return false;
-    sms_ = prop.multiProcessorCount;
+    // One attribute: the whole property table took 2.5 ms of a solve (up to 39).
+    if (!check(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_), "cudaDeviceGetAttribute")) return false;
     if (!check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
     for (cudaEvent_t& e : tev_)
         if (e == nullptr && !check(cudaEventCreate(&e), "cudaEventCreate")) return false;

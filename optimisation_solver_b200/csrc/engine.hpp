@@ -114,7 +114,7 @@ private:
     bool upload(void* dst, const void* src, size_t bytes) { return upload(dst, {{src, bytes}}); }
     // Device-to-host copy, complete on return.
     bool download(void* dst, const void* src, size_t bytes);
-    bool ensure_pinned();
+    bool ensure_pinned(size_t total);
     // Host phases of a solve, with PDLPGPU_TRACE=1 in the environment: the
     // seconds since the solve began at the end of each phase, printed to
     // stderr once the results are assembled.
@@ -169,6 +169,7 @@ private:
     int32_t* h_active_ = nullptr;     // pinned copy
     // two pinned staging buffers of large uploads and their last copies
     char* pinned_[2] = {nullptr, nullptr};
+    size_t pinned_chunk_ = 0;   // bytes of each
     cudaEvent_t pinned_done_[2] = {nullptr, nullptr};
     double device_seconds_ = 0.0;
     int64_t launches_ = 0;
