@@ -45,6 +45,26 @@ struct CtaWork {
     int32_t pad;
 };
 
+// All that a warp of a trial kernel needs to start on its first slice, in one
+// record per warp of the CTA map: following CTA map, instance and slice table
+// one after the other cost three round trips to L2 in every CTA.
+// Slots are counted in slices' units of 32; lines of all instances fit 32 bits
+// (each takes over a hundred bytes of device memory).
+struct alignas(16) WarpHead {
+    int32_t base;        // first slot of the slice / 32
+    int32_t line;        // its first line, in the space of all instances' lines
+    int32_t len;         // ... in the line lengths
+    int32_t other;       // the instance's first line of the other side
+    int32_t instance;
+    int32_t steps;
+    int32_t meta;        // as SliceDesc; no lines where the warp has no slice
+    int32_t slice;       // the slice, or slice_end
+    int32_t slice_end;   // of the CTA
+    int32_t many;        // the CTA has more slices than warps
+    int32_t pad[2];
+};
+static_assert(sizeof(WarpHead) == 48, "three 16-byte loads");
+
 struct VecWork {        // elementwise CTA: [begin, end) of one instance, rows or columns
     int32_t instance;
     int32_t is_row;

@@ -464,6 +464,8 @@ bool Engine::prepare(const SolveSpec& spec) {
     }
     plan.add(d_len, lens);
     plan.add(d_ctas, static_cast<int64_t>(a_ctas_.size() + at_ctas_.size()));
+    plan.add(g_.a.heads, kWarps * static_cast<int64_t>(a_ctas_.size()));
+    plan.add(g_.at.heads, kWarps * static_cast<int64_t>(at_ctas_.size()));
     plan.add(d_vec, static_cast<int64_t>(vec_.size()));
     plan.add(d_info, count_);
     plan.add(g_.ctl, count_);
@@ -482,7 +484,6 @@ bool Engine::prepare(const SolveSpec& spec) {
     plan.add(g_.part_dual, 2 * static_cast<int64_t>(a_ctas_.size()));
     plan.add(g_.part_prep, kPrepSlots * static_cast<int64_t>(vec_.size()));
     plan.add(g_.part_check, kCheckSlots * static_cast<int64_t>(a_ctas_.size() + at_ctas_.size()));
-    plan.add(g_.count_dual, count_);
     plan.add(g_.count_check, count_);
     plan.add(d_active_, 2);
     if (spec.ext.restart_metric == PDLPGPU_RESTART_NORMALIZED_GAP)
@@ -563,10 +564,13 @@ bool Engine::prepare(const SolveSpec& spec) {
         g_.vec = d_vec;
         g_.num_vec = static_cast<int32_t>(vec_.size());
         g_.info = d_info;
+        g_.instances = count_;
+        g_.sms = sms_;
         g_.shared_matrix = spec.shared_matrix ? 1 : 0;
         g_.mixed = mixed_ ? 1 : 0;
         g_.warm_x = nullptr;
         g_.warm_y = nullptr;
+        launch_warp_heads(g_, stream_);
         // A^T-side data bases, slice indices and line bases in info_ and in the
         // CTA map are relative to the g_.at pointers.
     }
@@ -867,7 +871,7 @@ template <class T>
 void Engine::enqueue_trial(const Work<T>& w) {
     launch_primal<T>(g_, w, dopt_, tuning_.vector_width, stream_);
     launch_dual<T>(g_, w, dopt_, tuning_.vector_width, stream_);
-    launches_ += 2;
+    launches_ += 3;
 }
 
 void Engine::enqueue_check_stage(bool il_sync) {
@@ -1037,20 +1041,20 @@ void Engine::enqueue_chunk(int slots, bool fp64_stage) {
             if (mixed_) launch_il_dual<float>(il32_, g_.ctl, dopt_, 0, k, stream_);
             else launch_il_dual<double>(il64_, g_.ctl, dopt_, 0, k, stream_);
         } else if (mixed_) {
-            launch_primal<float>(g_, w32_, dopt_, tuning_.vector_width, stream_);
+            launch_primal<float>(g_, w32_, dopt_, tuning_.vector_width, stream_, k > 0);
             if (p >= 0) record_timing(4 + 3 * p);
-            launch_dual<float>(g_, w32_, dopt_, tuning_.vector_width, stream_);
+            launch_dual<float>(g_, w32_, dopt_, tuning_.vector_width, stream_, true);
         } else {
-            launch_primal<double>(g_, w64_, dopt_, tuning_.vector_width, stream_);
+            launch_primal<double>(g_, w64_, dopt_, tuning_.vector_width, stream_, k > 0);
             if (p >= 0) record_timing(4 + 3 * p);
-            launch_dual<double>(g_, w64_, dopt_, tuning_.vector_width, stream_);
+            launch_dual<double>(g_, w64_, dopt_, tuning_.vector_width, stream_, true);
         }
-        launches_ += 2;
+        launches_ += il_ ? 2 : 3;
         if (p >= 0) record_timing(5 + 3 * p);
         if (mixed_ && fp64_stage) {
-            launch_primal<double>(g_, w64_, dopt_, tuning_.vector_width, stream_);
-            launch_dual<double>(g_, w64_, dopt_, tuning_.vector_width, stream_);
-            launches_ += 2;
+            launch_primal<double>(g_, w64_, dopt_, tuning_.vector_width, stream_, true);
+            launch_dual<double>(g_, w64_, dopt_, tuning_.vector_width, stream_, true);
+            launches_ += 3;
         }
     }
     record_timing(1);
@@ -1129,7 +1133,7 @@ bool Engine::build_graph(int slots, bool fp64_stage) {
 bool Engine::launch_chunk(int slots) {
     // h_active_[1]: instances in the FP64 stage at the last poll.
     const bool fp64 = mixed_ && h_active_[1] > 0;
-    const int trial_launches = fused_cluster_ > 0 ? (fp64 ? 2 : 1) : 2 * slots * (fp64 ? 2 : 1);
+    const int trial_launches = fused_cluster_ > 0 ? (fp64 ? 2 : 1) : (il_ ? 2 : 3) * slots * (fp64 ? 2 : 1);
     const int per_chunk = trial_launches + check_stage_launches(true);
     if (spec_.ext.disable_graphs) {
         enqueue_chunk(slots, fp64);

@@ -548,7 +548,7 @@ __device__ __forceinline__ void fused_decider(const DeviceOptions& o, InstanceCt
         trial_sync(C);
         trial_sync(C);
         const double* const sums_p = sums.p[t & 1];
-        // k_dual's fixed-order sums (warp_range_sums3: a lane's entries in
+        // k_dual's fixed-order sums (warp_range_sum_deep: a lane's entries in
         // order, then the butterfly; its steps that would only add the
         // zeros of lanes without entries are left out).
         double s[3], sp[1] = {0.0}, sd[2] = {0.0, 0.0};

@@ -6,8 +6,8 @@
 //             commit (iterate_average.cpp:40-82) while x is in registers.
 //   k_dual    over the A side: A x', extrapolation 2Ax' - Ax, dual prox
 //             y' = max(v - s u, 0) + min(v - s l, 0), sum dy^2/sigma and
-//             dy'(A dx); owed average update of y; then, in the last CTA of each
-//             instance, the linesearch decision and commit (trial_control).
+//             dy'(A dx); owed average update of y.
+//   k_decide  per instance: the linesearch decision and commit (trial_control).
 // Every check_frequency iterations (termination.cpp:66-325,
 // infeasibility.cpp:51-192, pdlp_solver.cpp:354-476), in FP64 on the original
 // problem:
@@ -184,44 +184,6 @@ __device__ __forceinline__ double warp_range_sum(const double* part, int begin, 
     return t;
 }
 
-// Warp-0 deterministic sums of three ranges of per-CTA partials at once:
-// every lane issues its loads of all three before the first add, so the
-// three reductions cost one round trip instead of three. Each result equals
-// warp_range_sum's for the same range (same per-lane order, same butterfly).
-template <bool kL2Only = false>
-__device__ __forceinline__ void warp_range_sums3(const double* p0, int b0, int e0, int s0, int q0,
-                                                 const double* p1, int b1, int e1, int s1, int q1,
-                                                 const double* p2, int b2, int e2, int s2, int q2,
-                                                 double (&out)[3]) {
-    const int lane = threadIdx.x & 31;
-    double t[3] = {0.0, 0.0, 0.0};
-    constexpr int kAhead = 4;   // partials per lane and range loaded at once
-    for (int k = 0;; k += 32 * kAhead) {
-        if (b0 + k >= e0 && b1 + k >= e1 && b2 + k >= e2) break;
-        double v[3][kAhead];
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const int o = k + 32 * u + lane;
-            auto get = [](const double* p) { return kL2Only ? __ldcg(p) : *p; };
-            v[0][u] = b0 + o < e0 ? get(p0 + static_cast<int64_t>(b0 + o) * s0 + q0) : 0.0;
-            v[1][u] = b1 + o < e1 ? get(p1 + static_cast<int64_t>(b1 + o) * s1 + q1) : 0.0;
-            v[2][u] = b2 + o < e2 ? get(p2 + static_cast<int64_t>(b2 + o) * s2 + q2) : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const int o = k + 32 * u + lane;
-            if (b0 + o < e0) t[0] += v[0][u];
-            if (b1 + o < e1) t[1] += v[1][u];
-            if (b2 + o < e2) t[2] += v[2][u];
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_xor_sync(kFull, t[q], o);
-        out[q] = t[q];
-    }
-}
-
 // Arrival counter: returns true in every thread of the CTA that arrives last
 // among `expected` CTAs of the instance (and resets the counter for the next
 // launch, which a kernel boundary orders). Partials written before the call
@@ -244,39 +206,47 @@ __device__ __forceinline__ bool arrive_last(int32_t* counter, int expected) {
 }
 
 
+// Programmatic dependent launch of the trial kernels (k_primal, k_dual,
+// k_decide): each lets its successor start as its own CTAs leave, and reads what
+// a trial kernel writes only after the wait, which returns once every earlier
+// kernel has ended and its writes are visible. Before it only data that no
+// trial kernel writes is read (heads, entries). Every CTA waits: a kernel's end
+// then means that all before it have ended.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Non-binding L2 prefetch of [p, p + bytes), shrunk inward to 16-byte
 // boundaries (so it never reaches outside the range) and cut into pieces of at
-// most 32 KiB spread over the CTA's threads starting at thread `first`.
-__device__ __forceinline__ void prefetch_range(const void* p, int64_t bytes, int first) {
+// most 32 KiB spread over the warp's lanes starting at lane `first`.
+__device__ __forceinline__ void prefetch_range(const void* p, int64_t bytes, int first, int lane) {
     if (bytes <= 0) return;
     const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15);
     const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + static_cast<uintptr_t>(bytes)) & ~uintptr_t(15);
     if (e <= a) return;
     constexpr uintptr_t kPiece = 32768;
     const uintptr_t pieces = (e - a + kPiece - 1) / kPiece;
-    for (uintptr_t k = (threadIdx.x + blockDim.x - static_cast<unsigned>(first) % blockDim.x) % blockDim.x;
-         k < pieces; k += blockDim.x) {
+    for (uintptr_t k = (static_cast<unsigned>(first) + lane) % 32; k < pieces; k += 32) {
         const uintptr_t b = a + k * kPiece;
         const uint32_t n = static_cast<uint32_t>(e - b < kPiece ? e - b : kPiece);
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b), "r"(n) : "memory");
     }
 }
 
-// The streams a SELL CTA reads once: its slices' index and value data and the
-// per-line vectors of its contiguous line range, prefetched into L2 when the
-// CTA starts, so its later slices find them there.
+// The streams of an entry with more slices than warps, prefetched into L2 by the
+// warp that starts its first record: its later slices find them there. `off`:
+// the instance's first line.
 template <class T, int NV>
-__device__ __forceinline__ void prefetch_cta(const Side& side, const CtaWork& cw, int64_t data_base,
-                                             const T* vals, const T* const (&vecs)[NV], int nvec) {
-    if (cw.slice_end <= cw.slice_begin) return;
-    const SliceDesc first = side.slices[cw.slice_begin], last = side.slices[cw.slice_end - 1];
+__device__ __forceinline__ void prefetch_entry(const Side& side, int slice_begin, int slice_end, int64_t data_base,
+                                               int64_t off, const T* vals, const T* const (&vecs)[NV], int nvec,
+                                               int lane) {
+    const SliceDesc first = side.slices[slice_begin], last = side.slices[slice_end - 1];
     const int64_t e0 = data_base + static_cast<int64_t>(first.data_off) * 32;
     const int64_t e1 = data_base + (static_cast<int64_t>(last.data_off) + last.steps) * 32;
-    prefetch_range(side.idx + e0, (e1 - e0) * 4, 0);
-    prefetch_range(vals + e0, (e1 - e0) * static_cast<int64_t>(sizeof(T)), 64);
-    const int l0 = first.line0, l1 = last.line0 + slice_lines(last.meta);
+    prefetch_range(side.idx + e0, (e1 - e0) * 4, 0, lane);
+    prefetch_range(vals + e0, (e1 - e0) * static_cast<int64_t>(sizeof(T)), 8, lane);
+    const int64_t l0 = off + first.line0, l1 = off + last.line0 + slice_lines(last.meta);
     for (int v = 0; v < nvec; ++v)
-        prefetch_range(vecs[v] + l0, static_cast<int64_t>(l1 - l0) * static_cast<int64_t>(sizeof(T)), 128 + 16 * v);
+        prefetch_range(vecs[v] + l0, (l1 - l0) * static_cast<int64_t>(sizeof(T)), 16 + 2 * v, lane);
 }
 
 __device__ __forceinline__ bool check_have_avg(const InstanceCtl& c, const DeviceOptions& o) {
@@ -292,8 +262,322 @@ template <> __device__ __forceinline__ const float* matrix_values<float>(const S
 // ---------------------------------------------------------------------------
 // Primal half (pdhg_kernel.cpp:47-104)
 // ---------------------------------------------------------------------------
+// ---------------------------------------------------------------------------
+// The trial kernels. A CTA takes every gridDim-th entry of the CTA map, as many
+// CTAs as the device holds at once. What starts an entry -- a record per warp
+// (WarpHead) and the instance's step (TrialParams) -- is brought into shared
+// memory for up to kTrialTile entries at once, and an entry's first slots and
+// indices are loaded while the gathers of the entry before it are in flight.
+//
+// Bound by latency: what a lane waits for is a gather of L2 under load (about
+// 2000 cycles). The random gathers alone would take 11 of the 38 us of a 200k x
+// 400k FP64 trial (290 G a second measured), its 90 MB of streams 12 at HBM's
+// rate. A CTA per entry, each following map, instance, slice table and slots one
+// after the other (14k cycles, three waves), and the decision in k_dual's last
+// CTA (21k cycles, its partials a round trip to L2 per 32) took 60 us; FP32, 48
+// LPs of 200 to 20000 rows: 52 -> 40 us.
+// ---------------------------------------------------------------------------
+constexpr int kTrialTile = 32;
+template <class T> constexpr int kTrialCtas = sizeof(T) == 8 ? 2 : 3;   // per SM: 128 and 80 registers a thread
+
+template <class T>
+struct alignas(16) TrialParams {
+    T mult;      // the half's step
+    T frac;      // of the pending average update
+    int32_t parity, pending, active;
+};
+
+template <class T>
+struct TrialShared {
+    WarpHead heads[kTrialTile][kWarps];
+    TrialParams<T> params[kTrialTile];
+    double red[kTrialTile][kWarps][2];   // a record's sums
+};
+
+// The tile's records: entries blockIdx.x + (t0 + i) gridDim.x, i < n.
+__device__ __forceinline__ void load_heads(const Side& side, int t0, int n, WarpHead (*heads)[kWarps]) {
+    constexpr int kWords = kWarps * static_cast<int>(sizeof(WarpHead) / 16);
+    for (int k = threadIdx.x; k < n * kWords; k += kThreads) {
+        const int64_t e = blockIdx.x + static_cast<int64_t>(t0 + k / kWords) * gridDim.x;
+        reinterpret_cast<int4*>(heads)[k] = __ldg(reinterpret_cast<const int4*>(side.heads + e * kWarps) + k % kWords);
+    }
+}
+
+// Lane i's entry of the tile: its instance's step, and whether it runs.
+template <class T, bool kDual>
+__device__ __forceinline__ TrialParams<T> trial_params(const Global& g, int instance) {
+    const InstanceCtl& c = g.ctl[instance];
+    TrialParams<T> k;
+    k.mult = static_cast<T>(kDual ? c.trial_eta * c.trial_omega : c.trial_eta / c.trial_omega);
+    k.frac = static_cast<T>(c.avg_frac);
+    k.parity = c.parity;
+    k.pending = !g.measure && c.pending_avg != 0;
+    k.active = g.measure || trial_active<T>(c);
+    return k;
+}
+
+// A lane's place in its warp's current slice.
+struct LineAt {
+    LanePos lp;
+    int steps, len;
+    int base, line;   // the slice's first slot / 32; the line in its whole space
+
+    __device__ __forceinline__ bool owner() const { return lp.valid && lp.g == 0; }
+    __device__ __forceinline__ int64_t slot0() const { return static_cast<int64_t>(base) * 32; }
+    __device__ __forceinline__ void at(const Side& side, int base32, int line0, int len0, int nsteps, int meta,
+                                       int lane) {
+        const SliceDesc sd{0, 0, nsteps, meta};
+        lp = lane_pos(sd, lane);
+        steps = nsteps;
+        base = base32;
+        line = line0 + lp.line;
+        len = lp.valid ? side.line_len[len0 + lp.line] : 0;
+    }
+    __device__ __forceinline__ void first(const Side& side, const WarpHead& h, int lane) {
+        at(side, h.base, h.line, h.len, h.steps, h.meta, lane);
+    }
+    // A later slice of the warp (CTAs with more slices than warps).
+    __device__ __forceinline__ void later(const Side& side, int64_t data_base, int64_t off, int64_t len_base,
+                                          int slice, int lane) {
+        const SliceDesc sd = side.slices[slice];
+        at(side, static_cast<int>(data_base / 32) + sd.data_off, static_cast<int>(off) + sd.line0,
+           static_cast<int>(len_base) + sd.line0, sd.steps, sd.meta, lane);
+    }
+};
+
+// A lane's entries in flight at once: four. With eight, which is a whole line for
+// a lane of all but the longest lines, FP64 spills at 128 registers (a trial of
+// 200k x 400k 40.3 us for 37.9) and FP32 has room for two CTAs an SM instead of
+// three (48 LPs of 200 to 20000 rows 41.3 us for 39.6).
+constexpr int kGroup = 4;
+template <class T>
+struct LineGroup {
+    int32_t id[kGroup];
+    T v[kGroup];
+
+    __device__ __forceinline__ void load(const Side& side, const T* vals, const LineAt& a, int s0, int lane) {
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) {
+            if (s0 + u < a.steps) {
+                const int64_t p = a.slot0() + static_cast<int64_t>(s0 + u) * 32 + lane;
+                id[u] = __ldg(side.idx + p);
+                v[u] = __ldg(vals + p);
+            }
+        }
+    }
+};
+
+// The line's product with the vector x, every lane of the line's group with the
+// same bits: line_sums from a loaded first group.
+template <class T>
+__device__ __forceinline__ T line_product(LineGroup<T>& group, const Side& side, const T* vals, const LineAt& a,
+                                          int lane, const T* x) {
+    // The lane has an entry in step s while (s << glog) + g < len.
+    const int mine = (a.len - a.lp.g + (1 << a.lp.glog) - 1) >> a.lp.glog;
+    T sum = T(0);
+    for (int s0 = 0;;) {
+        T xs[kGroup];
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u)
+            if (s0 + u < mine) xs[u] = x[group.id[u]];
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u)
+            if (s0 + u < mine) sum += group.v[u] * xs[u];
+        s0 += kGroup;
+        if (s0 >= a.steps) break;
+        group.load(side, vals, a, s0, lane);
+    }
+    for (int o = (1 << a.lp.glog) >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+    return sum;
+}
+
+// One half of a trial over the CTA's entries. `body(i, r, at, group, v)` runs the
+// slices of entry i's record r; its NR sums are added over the lanes at once,
+// over the entry's records in order at the end of the tile, and stored to
+// part[NR * entry + q]: the warps wait for one another once a tile, not once an
+// entry. A warp takes another record in each entry, since the last records of
+// many entries have no slice.
+template <class T, int NR, bool kDual, class Body>
+__device__ __forceinline__ void trial_half(const Global& g, const Side& side, TrialShared<T>& sh, double* part,
+                                           Body body) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const T* vals = matrix_values<T>(side);
+    const int mine = (side.num_ctas - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) /
+                     static_cast<int>(gridDim.x);
+    for (int t0 = 0; t0 < mine; t0 += kTrialTile) {
+        const int n = min(kTrialTile, mine - t0);
+        if (t0 > 0) __syncthreads();
+        load_heads(side, t0, n, sh.heads);
+        __syncthreads();
+        // The first entry is opened before it is known whether it runs.
+        LineAt at, next_at;
+        LineGroup<T> group, next_group;
+        auto record = [&](int i) { return (warp + 3 * i) % kWarps; };
+        auto open = [&](int i, LineAt& a, LineGroup<T>& gr) {
+            a.first(side, sh.heads[i][record(i)], lane);
+            gr.load(side, vals, a, 0, lane);
+        };
+        open(0, at, group);
+        if (t0 == 0) {
+            pdl_wait();
+            if (kDual) pdl_trigger();
+        }
+        if (static_cast<int>(threadIdx.x) < n)
+            sh.params[threadIdx.x] = trial_params<T, kDual>(g, sh.heads[threadIdx.x][0].instance);
+        __syncthreads();
+        const unsigned runs = __ballot_sync(kFull, lane < n && sh.params[lane].active != 0);
+        int i = __ffs(runs) - 1;
+        if (i > 0) open(i, at, group);
+        while (i >= 0) {
+            const int next = __ffs(runs & ~((2u << i) - 1u)) - 1;
+            if (next >= 0) open(next, next_at, next_group);
+            double v[NR];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) v[q] = 0.0;
+            const int r = record(i);
+            body(i, r, at, group, v);
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(kFull, v[q], o);
+                if (lane == 0) sh.red[i][r][q] = v[q];
+            }
+            i = next;
+            at = next_at;
+            group = next_group;
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < n * NR; k += kThreads) {
+            const int e = k / NR, q = k % NR;
+            if (!((runs >> e) & 1u)) continue;
+            double t = 0.0;
+            for (int w = 0; w < kWarps; ++w) t += sh.red[e][w][q];
+            part[NR * (blockIdx.x + static_cast<int64_t>(t0 + e) * gridDim.x) + q] = t;
+        }
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads, kTrialCtas<T>) k_primal(Global g, Work<T> w) {
+    __shared__ TrialShared<T> sh;
+    pdl_trigger();
+    const int lane = threadIdx.x & 31;
+    const T* vals = matrix_values<T>(g.at);
+    auto body = [&](int i, int r, LineAt& at, LineGroup<T>& group, double (&moved)[1]) {
+        const WarpHead& h = sh.heads[i][r];
+        const TrialParams<T> k = sh.params[i];
+        // Written by other kernels of the stream while this one may be
+        // waiting: no __restrict__.
+        const T* y = w.Y[k.parity] + h.other;
+        const T* x = w.X[k.parity];
+        T* xt = w.X[k.parity ^ 1];
+        T* avg = w.avg_x;
+        const InstanceInfo& inf = g.info[h.instance];
+        if (h.many && r == 0) {
+            const T* const vecs[7] = {x, w.c, w.xl, w.xu, w.tau, w.itau, avg};
+            prefetch_entry<T, 7>(g.at, h.slice, h.slice_end, inf.at_data_base, inf.col_off, vals, vecs,
+                                 k.pending ? 7 : 6, lane);
+        }
+        for (int s = h.slice; s < h.slice_end;) {
+            // The epilogue's operands do not depend on the product: loaded
+            // first, their latency overlaps the gathers'.
+            T cj = T(0), prev = T(0), loj = T(0), hij = T(0), tj = T(0), itj = T(0), aj = T(0);
+            if (at.owner()) {
+                cj = __ldg(w.c + at.line);
+                prev = x[at.line];
+                loj = __ldg(w.xl + at.line);
+                hij = __ldg(w.xu + at.line);
+                tj = __ldg(w.tau + at.line);
+                itj = __ldg(w.itau + at.line);
+                if (k.pending) aj = avg[at.line];
+            }
+            const T sum = line_product(group, g.at, vals, at, lane, y);
+            if (at.owner()) {
+                const T gradient = cj + sum;
+                const T upd = smax(loj, smin(prev - k.mult * tj * gradient, hij));
+                xt[at.line] = upd;
+                const double d = static_cast<double>(upd - prev);
+                moved[0] += d * d * static_cast<double>(itj);
+                if (k.pending) avg[at.line] = aj + k.frac * (prev - aj);
+            }
+            s += kWarps;
+            if (s < h.slice_end) {
+                at.later(g.at, inf.at_data_base, inf.col_off, inf.at_len_base, s, lane);
+                group.load(g.at, vals, at, 0, lane);
+            }
+        }
+    };
+    trial_half<T, 1, false>(g, g.at, sh, g.part_primal, body);
+}
+
+// ---------------------------------------------------------------------------
+// Dual half (pdhg_kernel.cpp:109-187) and the trial decision
+// ---------------------------------------------------------------------------
+template <class T>
+__global__ void __launch_bounds__(kThreads, kTrialCtas<T>) k_dual(Global g, Work<T> w) {
+    __shared__ TrialShared<T> sh;
+    const int lane = threadIdx.x & 31;
+    const T* vals = matrix_values<T>(g.a);
+    auto body = [&](int i, int r, LineAt& at, LineGroup<T>& group, double (&red)[2]) {
+        const WarpHead& h = sh.heads[i][r];
+        const TrialParams<T> k = sh.params[i];
+        const T* xt = w.X[k.parity ^ 1] + h.other;
+        const T* y = w.Y[k.parity];
+        T* yt = w.Y[k.parity ^ 1];
+        const T* ax = w.AX[k.parity];
+        T* axt = w.AX[k.parity ^ 1];
+        T* avg = w.avg_y;
+        const InstanceInfo& inf = g.info[h.instance];
+        if (h.many && r == 0) {
+            const T* const vecs[7] = {ax, y, w.rl, w.ru, w.sigma, w.isigma, avg};
+            prefetch_entry<T, 7>(g.a, h.slice, h.slice_end, inf.a_data_base, inf.row_off, vals, vecs,
+                                 k.pending ? 7 : 6, lane);
+        }
+        for (int s = h.slice; s < h.slice_end;) {
+            T axi = T(0), sgi = T(0), prev = T(0), loi = T(0), hii = T(0), isi = T(0), ai = T(0);
+            if (at.owner()) {
+                axi = ax[at.line];
+                sgi = __ldg(w.sigma + at.line);
+                prev = y[at.line];
+                loi = __ldg(w.rl + at.line);
+                hii = __ldg(w.ru + at.line);
+                isi = __ldg(w.isigma + at.line);
+                if (k.pending) ai = avg[at.line];
+            }
+            const T sum = line_product(group, g.a, vals, at, lane, xt);
+            if (at.owner()) {
+                const T next = sum;
+                const T dact = next - axi;
+                const T ext = next + dact;
+                const T step = smax(k.mult * sgi, min_dual_step<T>());
+                const T v = prev + step * ext;
+                const T upd = smax(v - step * hii, T(0)) + smin(v - step * loi, T(0));
+                yt[at.line] = upd;
+                axt[at.line] = next;
+                const double d = static_cast<double>(upd - prev);
+                red[0] += d * d * static_cast<double>(isi);
+                red[1] += d * static_cast<double>(dact);
+                if (k.pending) avg[at.line] = ai + k.frac * (prev - ai);
+            }
+            s += kWarps;
+            if (s < h.slice_end) {
+                at.later(g.a, inf.a_data_base, inf.row_off, inf.a_len_base, s, lane);
+                group.load(g.a, vals, at, 0, lane);
+            }
+        }
+    };
+    trial_half<T, 2, true>(g, g.a, sh, g.part_dual, body);
+}
+
+// The two halves for long lines (V > 1: a mean of 12 entries, FP64 16, or more): a
+// CTA per entry, four an SM, its slots streamed V at a time with a group ahead.
+// Such matrices are streams more than gathers, and the bytes in flight count: on
+// 1024 LPs of 200 to 50000 rows (145M entries, FP32, V = 4) these take 525 and
+// 504 us where the kernels above, at two CTAs an SM, took 643 and 588.
 template <class T, int V>
-__global__ void __launch_bounds__(kThreads, 4) k_primal(Global g, Work<T> w) {
+__global__ void __launch_bounds__(kThreads, 4) k_primal_wide(Global g, Work<T> w) {
+    pdl_trigger();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const CtaWork cw = g.at.ctas[blockIdx.x];
     const InstanceCtl& c = g.ctl[cw.instance];
     if (!g.measure && !trial_active<T>(c)) return;
@@ -303,8 +587,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_primal(Global g, Work<T> w) {
     const bool pending = !g.measure && c.pending_avg != 0;
     const T frac = static_cast<T>(c.avg_frac);
 
-    const T* __restrict__ y = w.Y[p] + inf.row_off;
-    const T* __restrict__ x = w.X[p] + inf.col_off;
+    const T* y = w.Y[p] + inf.row_off;
+    const T* x = w.X[p] + inf.col_off;
     T* __restrict__ xt = w.X[p ^ 1] + inf.col_off;
     const T* __restrict__ cv = w.c + inf.col_off;
     const T* __restrict__ lo = w.xl + inf.col_off;
@@ -315,11 +599,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_primal(Global g, Work<T> w) {
     const T* vals = matrix_values<T>(g.at);
     {
         const T* const vecs[7] = {x, cv, lo, hi, tau, itau, avg};
-        prefetch_cta<T, 7>(g.at, cw, inf.at_data_base, vals, vecs, pending ? 7 : 6);
+        if (warp == 0 && cw.slice_end > cw.slice_begin)
+            prefetch_entry<T, 7>(g.at, cw.slice_begin, cw.slice_end, inf.at_data_base, 0, vals, vecs, pending ? 7 : 6, lane);
     }
 
     double moved[1] = {0.0};
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int s = cw.slice_begin + warp; s < cw.slice_end; s += kWarps) {
         const SliceDesc sd = g.at.slices[s];
         const LanePos lp = lane_pos(sd, lane);
@@ -355,11 +639,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_primal(Global g, Work<T> w) {
     if (threadIdx.x == 0) g.part_primal[blockIdx.x] = moved[0];
 }
 
-// ---------------------------------------------------------------------------
-// Dual half (pdhg_kernel.cpp:109-187) and the trial decision
-// ---------------------------------------------------------------------------
 template <class T, int V>
-__global__ void __launch_bounds__(kThreads, 4) k_dual(Global g, Work<T> w, DeviceOptions o) {
+__global__ void __launch_bounds__(kThreads, 4) k_dual_wide(Global g, Work<T> w) {
+    pdl_wait();
+    pdl_trigger();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const CtaWork cw = g.a.ctas[blockIdx.x];
     InstanceCtl& c = g.ctl[cw.instance];
     if (!g.measure && !trial_active<T>(c)) return;
@@ -369,10 +653,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_dual(Global g, Work<T> w, Devic
     const bool pending = !g.measure && c.pending_avg != 0;
     const T frac = static_cast<T>(c.avg_frac);
 
-    const T* __restrict__ xt = w.X[p ^ 1] + inf.col_off;
-    const T* __restrict__ y = w.Y[p] + inf.row_off;
+    const T* xt = w.X[p ^ 1] + inf.col_off;
+    const T* y = w.Y[p] + inf.row_off;
     T* __restrict__ yt = w.Y[p ^ 1] + inf.row_off;
-    const T* __restrict__ ax = w.AX[p] + inf.row_off;
+    const T* ax = w.AX[p] + inf.row_off;
     T* __restrict__ axt = w.AX[p ^ 1] + inf.row_off;
     const T* __restrict__ lo = w.rl + inf.row_off;
     const T* __restrict__ hi = w.ru + inf.row_off;
@@ -382,11 +666,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_dual(Global g, Work<T> w, Devic
     const T* vals = matrix_values<T>(g.a);
     {
         const T* const vecs[7] = {ax, y, lo, hi, sig, isig, avg};
-        prefetch_cta<T, 7>(g.a, cw, inf.a_data_base, vals, vecs, pending ? 7 : 6);
+        if (warp == 0 && cw.slice_end > cw.slice_begin)
+            prefetch_entry<T, 7>(g.a, cw.slice_begin, cw.slice_end, inf.a_data_base, 0, vals, vecs, pending ? 7 : 6, lane);
     }
 
     double red[2] = {0.0, 0.0};
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int s = cw.slice_begin + warp; s < cw.slice_end; s += kWarps) {
         const SliceDesc sd = g.a.slices[s];
         const LanePos lp = lane_pos(sd, lane);
@@ -427,34 +711,71 @@ __global__ void __launch_bounds__(kThreads, 4) k_dual(Global g, Work<T> w, Devic
         g.part_dual[2 * blockIdx.x] = red[0];
         g.part_dual[2 * blockIdx.x + 1] = red[1];
     }
-    if (g.measure) return;
-    // Whichever CTA turns out last decides: each brings the instance's
-    // control block into its L1 while the arrival is in flight, so the
-    // decision's reads of it do not each wait on L2.
-    if (threadIdx.x < sizeof(InstanceCtl) / 128)
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char*>(&c) + 128 * threadIdx.x));
-    if (!arrive_last(g.count_dual + cw.instance, inf.a_cta_end - inf.a_cta_begin)) return;
-    // Options by reference from shared memory (a reference to the kernel
-    // parameter would copy it to local memory in every thread).
-    __shared__ DeviceOptions so;
-    if (threadIdx.x == 0) so = o;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        // The decision runs on a shared-memory copy of the control block:
-        // after a store to a global line, the thread's next load of that line
-        // would be served by L2, and the decision reads back much of what it
-        // writes.
-        __shared__ alignas(16) InstanceCtl sc;
-        copy_ctl_warp(&sc, &c);
-        double sums[3];
-        warp_range_sums3(g.part_primal, inf.at_cta_begin, inf.at_cta_end, 1, 0,
-                         g.part_dual, inf.a_cta_begin, inf.a_cta_end, 2, 0,
-                         g.part_dual, inf.a_cta_begin, inf.a_cta_end, 2, 1, sums);
-        __syncwarp();
-        if (threadIdx.x == 0) trial_control(sc, so, sums[0], sums[1], sums[2], inf.n);
-        __syncwarp();
-        copy_ctl_warp(&c, &sc);
+}
+
+// warp_range_sum with up to 16 of a lane's partials in flight.
+__device__ __forceinline__ double warp_range_sum_deep(const double* part, int begin, int end, int slots, int slot) {
+    constexpr int kAhead = 16;
+    const int lane = threadIdx.x & 31;
+    double t = 0.0;
+    for (int k = begin + lane; k < end; k += 32 * kAhead) {
+        double v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            v[u] = k + 32 * u < end ? part[static_cast<int64_t>(k + 32 * u) * slots + slot] : 0.0;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (k + 32 * u < end) t += v[u];
     }
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+    return t;
+}
+
+// The decision on a trial, a CTA per instance: the entries' partials are added
+// in a fixed order, a warp per sum, then trial_control runs on a shared-memory
+// copy of the control block (after a store to a global line the thread's next
+// load of that line would be served by L2, and the decision reads back much of
+// what it writes). The control block, the options (by reference from shared
+// memory: a reference to the kernel parameter would copy it to local memory in
+// every thread) and the step factors are there before the wait: only the
+// previous decision writes the block, and k_dual lets this kernel start after
+// its own wait, when that decision has ended.
+constexpr int kDecideThreads = 96;
+template <class T>
+__global__ void __launch_bounds__(kDecideThreads) k_decide(Global g, DeviceOptions o) {
+    __shared__ DeviceOptions so;
+    __shared__ alignas(16) InstanceCtl sc;
+    __shared__ double factors[2];
+    __shared__ double sums[3];
+    pdl_trigger();
+    InstanceCtl* c = g.ctl + blockIdx.x;
+    const InstanceInfo& inf = g.info[blockIdx.x];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = inf.n;
+    const int begin = warp == 0 ? inf.at_cta_begin : inf.a_cta_begin;
+    const int end = warp == 0 ? inf.at_cta_end : inf.a_cta_end;
+    bool have = false;
+    if (warp == 0) {
+        if (lane < static_cast<int>(sizeof(InstanceCtl) / 16))
+            reinterpret_cast<int4*>(&sc)[lane] = __ldcg(reinterpret_cast<const int4*>(c) + lane);
+        __syncwarp();
+        const int64_t k = sc.phase == kPhasePolish ? sc.polish_iteration : sc.iteration;
+        have = k >= 0 && k < o.step_pow_entries;
+        if (have && lane < 2) factors[lane] = __ldg(o.step_pow + 2 * k + lane);
+    } else if (warp == 1 && lane == 0) {
+        so = o;
+    }
+    pdl_wait();
+    __syncthreads();
+    if (!trial_active<T>(sc)) return;
+    const double t = warp_range_sum_deep(warp == 0 ? g.part_primal : g.part_dual, begin, end, warp == 0 ? 1 : 2,
+                                         warp == 2 ? 1 : 0);
+    if (lane == 0) sums[warp] = t;
+    __syncthreads();
+    if (warp != 0) return;
+    if (lane == 0) trial_control(sc, so, sums[0], sums[1], sums[2], n, have ? factors : nullptr);
+    __syncwarp();
+    copy_ctl_warp(c, &sc);
 }
 
 // Fused trials of small LPs (k_fused).
@@ -952,7 +1273,7 @@ __global__ void __launch_bounds__(kThreads) k_check_spmv(Global g, DeviceOptions
     if (!arrive_last(g.count_check + cw.instance, expected)) return;
     // With normalised-gap restarts, k_check_ndg takes the decision.
     if (o.ndg_restarts) return;
-    __shared__ DeviceOptions so;   // see k_dual
+    __shared__ DeviceOptions so;   // see k_decide
     if (threadIdx.x == 0) so = o;
     __syncthreads();
     if (threadIdx.x < 32) check_control(g, so, c, inf, nullptr);
@@ -966,7 +1287,7 @@ __global__ void __launch_bounds__(kThreads) k_check_ndg(Global g, DeviceOptions 
     InstanceCtl& c = g.ctl[b];
     if (c.stage != kStageCheck || c.check_kind == kCheckTransition) return;
     const InstanceInfo inf = g.info[b];
-    __shared__ DeviceOptions so;   // see k_dual
+    __shared__ DeviceOptions so;   // see k_decide
     __shared__ double gaps[2];
     if (threadIdx.x == 0) so = o;
     __syncthreads();
@@ -1219,6 +1540,32 @@ __device__ __forceinline__ double initial_value(double lo, double hi) {   // pdl
     if (isfinite(lo)) return lo;
     if (isfinite(hi)) return hi;
     return 0.0;
+}
+
+__global__ void k_warp_heads(Global g) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool a_side = k < g.a.num_ctas * kWarps;
+    const int i = a_side ? k : k - g.a.num_ctas * kWarps;
+    const Side& side = a_side ? g.a : g.at;
+    if (i >= side.num_ctas * kWarps) return;
+    const CtaWork cw = side.ctas[i / kWarps];
+    const InstanceInfo inf = g.info[cw.instance];
+    const int s = cw.slice_begin + i % kWarps;
+    const bool some = s < cw.slice_end;
+    SliceDesc sd{};
+    if (some) sd = side.slices[s];
+    WarpHead h{};
+    h.base = static_cast<int32_t>((a_side ? inf.a_data_base : inf.at_data_base) / 32) + sd.data_off;
+    h.line = static_cast<int32_t>(a_side ? inf.row_off : inf.col_off) + sd.line0;
+    h.len = static_cast<int32_t>(a_side ? inf.a_len_base : inf.at_len_base) + sd.line0;
+    h.other = static_cast<int32_t>(a_side ? inf.col_off : inf.row_off);
+    h.instance = cw.instance;
+    h.steps = sd.steps;
+    h.meta = sd.meta;
+    h.slice = some ? s : cw.slice_end;
+    h.slice_end = cw.slice_end;
+    h.many = cw.slice_end - cw.slice_begin > kWarps;
+    side.heads[i] = h;
 }
 
 // Scaled objective and bounds (scaling.cpp:109-135), the starting point
@@ -1560,13 +1907,41 @@ inline unsigned blocks_for(int64_t n, int per) { return static_cast<unsigned>((n
 // ---------------------------------------------------------------------------
 // Launch wrappers
 // ---------------------------------------------------------------------------
+void launch_warp_heads(const Global& g, cudaStream_t s) {
+    const int64_t n = static_cast<int64_t>(g.a.num_ctas + g.at.num_ctas) * kWarps;
+    if (n > 0) k_warp_heads<<<blocks_for(n, 256), 256, 0, s>>>(g);
+}
+
+namespace {
+// A trial kernel; `chained`: its predecessor in the stream is a trial kernel,
+// so it may start while that one ends (see pdl_wait).
+template <class... P, class... A>
+void launch_trial(void (*kernel)(P...), int32_t ctas, int threads, bool chained, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+// As many CTAs as the device holds at once, at most one per entry of the map.
 template <class T>
-void launch_primal(const Global& g, const Work<T>& w, const DeviceOptions&, int vw, cudaStream_t s) {
+int32_t trial_ctas(const Global& g, const Side& side) {
+    return std::min<int32_t>(side.num_ctas, g.sms * kTrialCtas<T>);
+}
+}  // namespace
+
+template <class T>
+void launch_primal(const Global& g, const Work<T>& w, const DeviceOptions&, int vw, cudaStream_t s, bool chained) {
     if (g.at.num_ctas == 0) return;
     switch (vw) {
-        case 4: k_primal<T, 4><<<g.at.num_ctas, kThreads, 0, s>>>(g, w); break;
-        case 2: k_primal<T, 2><<<g.at.num_ctas, kThreads, 0, s>>>(g, w); break;
-        default: k_primal<T, 1><<<g.at.num_ctas, kThreads, 0, s>>>(g, w); break;
+        case 4: launch_trial(k_primal_wide<T, 4>, g.at.num_ctas, kThreads, chained, s, g, w); break;
+        case 2: launch_trial(k_primal_wide<T, 2>, g.at.num_ctas, kThreads, chained, s, g, w); break;
+        default: launch_trial(k_primal<T>, trial_ctas<T>(g, g.at), kThreads, chained, s, g, w); break;
     }
 }
 
@@ -1643,13 +2018,15 @@ int fused_max_clusters(int vw, int cluster, const FusedShape& shape) {
 }
 
 template <class T>
-void launch_dual(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw, cudaStream_t s) {
+void launch_dual(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw, cudaStream_t s,
+                 bool chained) {
     if (g.a.num_ctas == 0) return;
     switch (vw) {
-        case 4: k_dual<T, 4><<<g.a.num_ctas, kThreads, 0, s>>>(g, w, o); break;
-        case 2: k_dual<T, 2><<<g.a.num_ctas, kThreads, 0, s>>>(g, w, o); break;
-        default: k_dual<T, 1><<<g.a.num_ctas, kThreads, 0, s>>>(g, w, o); break;
+        case 4: launch_trial(k_dual_wide<T, 4>, g.a.num_ctas, kThreads, chained, s, g, w); break;
+        case 2: launch_trial(k_dual_wide<T, 2>, g.a.num_ctas, kThreads, chained, s, g, w); break;
+        default: launch_trial(k_dual<T>, trial_ctas<T>(g, g.a), kThreads, chained, s, g, w); break;
     }
+    if (!g.measure) launch_trial(k_decide<T>, g.instances, kDecideThreads, true, s, g, o);
 }
 
 template <class T>
@@ -1838,11 +2215,11 @@ void launch_slot_done(const Global& g, int32_t count, int32_t* done, cudaStream_
 }
 
 #define PDLPGPU_INSTANTIATE(T)                                                                      \
-    template void launch_primal<T>(const Global&, const Work<T>&, const DeviceOptions&, int, cudaStream_t); \
+    template void launch_primal<T>(const Global&, const Work<T>&, const DeviceOptions&, int, cudaStream_t, bool); \
     template cudaError_t launch_fused<T>(const Global&, const Work<T>&, const DeviceOptions&, int, int, int, \
                                          int, const FusedShape&, cudaStream_t);                      \
     template int fused_max_clusters<T>(int, int, const FusedShape&);                                 \
-    template void launch_dual<T>(const Global&, const Work<T>&, const DeviceOptions&, int, cudaStream_t);   \
+    template void launch_dual<T>(const Global&, const Work<T>&, const DeviceOptions&, int, cudaStream_t, bool); \
     template void launch_check_prep<T>(const Global&, const Work<T>&, const DeviceOptions&, cudaStream_t);  \
     template void launch_check_apply<T>(const Global&, const Work<T>&, const DeviceOptions&, cudaStream_t); \
     template void launch_refresh<T>(const Global&, const Work<T>&, const DeviceOptions&, int, cudaStream_t); \

@@ -16,6 +16,7 @@ struct Side {
     const float* val_s32;        // Ruiz-scaled coefficients (FP32), mixed precision only
     const int32_t* line_len;
     const CtaWork* ctas;
+    WarpHead* heads;             // [num_ctas][kWarps]
     int32_t num_ctas;
 };
 
@@ -47,6 +48,8 @@ struct Global {
     Side a, at;
     const VecWork* vec;
     int32_t num_vec;
+    int32_t instances;           // on the device
+    int32_t sms;                 // the device's SMs
     int32_t shared_matrix;
     // original problem (FP64) and the Ruiz scale vectors
     double* rs;
@@ -73,12 +76,11 @@ struct Global {
     // setup scratch
     double* row_tmp;
     double* col_tmp;
-    // per-CTA partials and per-instance arrival counters
+    // per-CTA partials and per-instance arrival counters of the checks
     double* part_primal;
     double* part_dual;
     double* part_prep;
     double* part_check;
-    int32_t* count_dual;
     int32_t* count_check;
     // 1: timing mode -- every instance runs its trial kernels, no decision is
     // taken and no state changes (the trial buffers are scratch).
@@ -101,12 +103,18 @@ struct Global {
 
 // --- launches (kernels.cu). `vw` is the vector width (1, 2 or 4). ---------
 
+// Fills both sides' WarpHead tables from the CTA map, the slices and the
+// instances.
+void launch_warp_heads(const Global& g, cudaStream_t s);
+// The two halves of a trial, the second with the decision (outside timing
+// mode). `chained`: the kernel before this one in the stream is one of theirs,
+// whose end it may then overlap.
 template <class T>
 void launch_primal(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw,
-                   cudaStream_t s);
+                   cudaStream_t s, bool chained = false);
 template <class T>
 void launch_dual(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw,
-                 cudaStream_t s);
+                 cudaStream_t s, bool chained = false);
 // Where a fused launch keeps its vectors (fused.cuh).
 enum : int32_t { kFusedGlobal = 0, kFusedStaged = 1, kFusedHalf = 2, kFusedCopies = 3 };
 // The shape of a fused launch's shared memory, over its instances.
