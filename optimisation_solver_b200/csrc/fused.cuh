@@ -34,7 +34,7 @@
 // the barrier's release and acquire order them.
 //
 // Bound by latency: two cluster barriers and three dependent phases a trial.
-// 100 trials, FP64, of a 64 x 128 planted LP (one CTA) 224 us, 1000 x 2000
+// 100 trials, FP64, of a 40 x 70 planted LP (one CTA) 224 us, 1000 x 2000
 // (4 CTAs) 409, a 2000-node flow LP (16 CTAs, half) 863. With three barriers a
 // trial, the decision by the workers and 32-bit indices from step-major global
 // slices they were 383, 570 and 1133. Of 1000 x 2000's 7800 cycles a trial

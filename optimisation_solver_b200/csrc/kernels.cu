@@ -270,12 +270,12 @@ template <> __device__ __forceinline__ const float* matrix_values<float>(const S
 // indices are loaded while the gathers of the entry before it are in flight.
 //
 // Bound by latency: what a lane waits for is a gather of L2 under load (about
-// 2000 cycles). The random gathers alone would take 11 of the 38 us of a 200k x
-// 400k FP64 trial (290 G a second measured), its 90 MB of streams 12 at HBM's
-// rate. A CTA per entry, each following map, instance, slice table and slots one
-// after the other (14k cycles, three waves), and the decision in k_dual's last
-// CTA (21k cycles, its partials a round trip to L2 per 32) took 60 us; FP32, 48
-// LPs of 200 to 20000 rows: 52 -> 40 us.
+// 2000 cycles). Of the 38 us of a 200k x 400k FP64 trial (2M entries) the random
+// gathers alone would take 14 (285 G a second measured), its 93 MB of streams 14
+// at HBM's rate. A CTA per entry, each following map, instance, slice table and
+// slots one after the other (14k cycles, three waves), and the decision in
+// k_dual's last CTA (21k cycles, its partials a round trip to L2 per 32) took
+// 60 us; FP32, 48 LPs of 200 to 20000 rows: 51 -> 40 us.
 // ---------------------------------------------------------------------------
 constexpr int kTrialTile = 32;
 template <class T> constexpr int kTrialCtas = sizeof(T) == 8 ? 2 : 3;   // per SM: 128 and 80 registers a thread
