@@ -127,10 +127,10 @@ constexpr size_t kPinnedMin = size_t(4) << 20;      // bytes per staging buffer
 constexpr size_t kPinnedMax = size_t(64) << 20;
 constexpr size_t kPinnedDirect = size_t(4) << 20;   // smaller uploads go as they are
 
-// Host memcpy piece per thread: about 16 of a chunk, so that a small chunk has
-// as many threads copying as the memory needs.
+// Host memcpy piece per thread: up to 16 of a chunk, and none below 1 MiB, where
+// starting a thread costs as much as the copy.
 size_t copy_job(size_t chunk) {
-    return std::min(std::max(chunk / 16, size_t(256) << 10), size_t(2) << 20);
+    return std::min(std::max(chunk / 16, size_t(1) << 20), size_t(2) << 20);
 }
 }  // namespace
 
