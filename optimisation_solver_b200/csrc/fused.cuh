@@ -232,8 +232,9 @@ __device__ __forceinline__ void store_copies(const T* elem, T v, uint32_t C) {
     for (uint32_t r = 0; r < C; ++r) st_cluster(rank_addr(elem, r), v);
 }
 
-// Step factors a launch keeps in shared memory (trials past them take the
-// slow decision, which reads the options' table).
+// Step factors a CTA keeps in shared memory, of the iteration indices that come
+// next; trials past them fetch as many again (past the options' table the
+// slow decision computes them).
 constexpr int kFusedFactors = 160;
 __device__ __forceinline__ int fused_factors(const DeviceOptions& o, int64_t first) {
     const int64_t avail = first >= 0 && first < o.step_pow_entries ? o.step_pow_entries - first : 0;
@@ -249,7 +250,7 @@ struct FusedState {
     double eta, omega_eval, omega_trial, eta_max;   // of the phase's controller
     double avg_weight, avg_frac;
     double sums[3];
-    int64_t index0;       // iteration index at load; factors are relative to it
+    int64_t index0;       // iteration index at load
     int64_t to_check;     // accepted trials until the check boundary or the limit
     int parity, pending, rejected;
     int accepted, trials; // since the load
@@ -302,13 +303,17 @@ struct FusedState {
         c.trials_this_iter = rejected;
     }
 
+    // Iteration index of the trial under way.
+    __device__ __forceinline__ int64_t iteration() const { return index0 + accepted; }
+
+    // `factors`: nfactors of them, from iteration index `first` on.
     __device__ __forceinline__ bool decide(const DeviceOptions& o, const double (&s)[3], const double* factors,
-                                           int nfactors) {
-        const int64_t k = accepted;   // iteration index, relative to index0
+                                           int64_t first, int nfactors) {
+        const int64_t k = iteration() - first;
         if (!plain || k >= nfactors || !(isfinite(s[0]) && isfinite(s[1]) && isfinite(s[2]))) return false;
         double next = eta;
         const bool accept =
-            evaluate_step(next, omega_eval, eta_max, o, s[0], s[1], s[2], index0 + k, factors + 2 * k);
+            evaluate_step(next, omega_eval, eta_max, o, s[0], s[1], s[2], iteration(), factors + 2 * k);
         if (accept ? to_check <= 1 : rejected + 1 >= o.max_trials) return false;
         eta = next;
         ++trials;
@@ -474,7 +479,6 @@ struct FusedCta {
     DeviceOptions so;
     FusedCtl f;
     InstanceCtl ctl;
-    // step_pow entries of iteration indices from the launch's first on.
     double fac[2 * kFusedFactors];
 };
 struct FusedRange {
@@ -520,31 +524,34 @@ __device__ __forceinline__ FusedRange fused_setup(const Global& g, const DeviceO
         const CtaWork cw = g.a.ctas[inf.a_cta_begin + e];
         sums.tab_d[e] = ((cw.slice_begin - r.ds0) << 4) | (cw.slice_end - cw.slice_begin);
     }
-    // The linesearch's step factors of the launch's iteration indices (one
-    // phase per launch: a phase ends at a check, which ends the launch).
-    const int64_t fac0 = cp->phase == kPhasePolish ? cp->polish_iteration : cp->iteration;
-    const int n = fused_factors(o, fac0);
-    for (int q = threadIdx.x; q < 2 * n; q += kFusedThreads) sc.fac[q] = o.step_pow[2 * fac0 + q];
     return r;
 }
 
 // The deciding warp of a CTA, from the first trial to the launch's end.
-__device__ __forceinline__ void fused_decider(const DeviceOptions& o, InstanceCtl* cp, int32_t n_cols, bool fp64,
-                                              int max_trials, FusedCta& sc, const FusedSums& sums,
-                                              const FusedRange& range, uint32_t C, uint32_t rank) {
+__device__ __forceinline__ void fused_decider(InstanceCtl* cp, int32_t n_cols, bool fp64, int max_trials,
+                                              FusedCta& sc, const FusedSums& sums, const FusedRange& range,
+                                              uint32_t C, uint32_t rank) {
     const int lane = threadIdx.x & 31;
     DeviceOptions& so = sc.so;
     FusedCtl& f = sc.f;
     InstanceCtl& sctl = sc.ctl;
-    const int64_t fac0 = sctl.phase == kPhasePolish ? sctl.polish_iteration : sctl.iteration;
-    const int nfac = fused_factors(o, fac0);
     // Its registers are never the workers'; its barriers match theirs one for
     // one.
     FusedState state;
     state.load(sctl, so);
+    int64_t fac0 = 0;   // the factors kept are of iteration indices fac0, fac0 + 1, ..., nfac of them
+    int nfac = 0;
     int widest = 16;   // the butterfly's first step that meets an entry
     while (widest > 0 && widest >= max(range.ne_p, range.ne_d)) widest >>= 1;
     for (int t = 0; t < max_trials && f.active; ++t) {
+        // By index, not by trial: a slow decision inside an interval loads the
+        // state anew, past the iteration that the launch began with.
+        if (state.iteration() - fac0 >= nfac) {
+            fac0 = state.iteration();
+            nfac = fused_factors(so, fac0);
+            for (int q = lane; q < 2 * nfac; q += 32) sc.fac[q] = so.step_pow[2 * fac0 + q];
+            __syncwarp();
+        }
         trial_sync(C);
         trial_sync(C);
         const double* const sums_p = sums.p[t & 1];
@@ -564,7 +571,7 @@ __device__ __forceinline__ void fused_decider(const DeviceOptions& o, InstanceCt
 #pragma unroll
         for (int q = 0; q < 3; ++q) s[q] = __shfl_sync(kFull, s[q], 0);
         const int before = state.accepted;
-        if (state.decide(so, s, sc.fac, nfac)) {
+        if (state.decide(so, s, sc.fac, fac0, nfac)) {
             if (lane == 0) {
                 f.mult_primal = state.eta / state.omega_trial;
                 f.mult_dual = state.eta * state.omega_trial;
@@ -578,9 +585,7 @@ __device__ __forceinline__ void fused_decider(const DeviceOptions& o, InstanceCt
             if (rank == 0) {
                 if (lane == 0) {
                     state.store(sctl, so);
-                    const int64_t k = sctl.phase == kPhasePolish ? sctl.polish_iteration : sctl.iteration;
-                    const double* fk = k >= fac0 && k - fac0 < nfac ? sc.fac + 2 * (k - fac0) : nullptr;
-                    trial_control(sctl, so, s[0], s[1], s[2], n_cols, fk);
+                    trial_control(sctl, so, s[0], s[1], s[2], n_cols);
                 }
                 __syncwarp();
                 if (lane < static_cast<int>(sizeof(InstanceCtl) / 16)) {
@@ -702,7 +707,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w,
     // Remote shared memory is written only once every CTA of the cluster runs.
     cluster_sync_all();
     if (decider) {
-        fused_decider(o, cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
+        fused_decider(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
         return;
     }
 
@@ -880,7 +885,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused_global(Global g, Wor
     if (decider && lane == 0) fused_snapshot(sc.ctl, f, kFp64);
     cluster_sync_all();
     if (decider) {
-        fused_decider(o, cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
+        fused_decider(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
         return;
     }
     auto publish = [&](double* at, double v) {
