@@ -459,7 +459,7 @@ struct pdlpgpu_mlp {
     };
     Report *report_dev = nullptr, *report = nullptr;
     int* err = nullptr;         // &report_dev->err
-    int64_t step = 0;
+    int64_t step = 0;           // Adam steps taken
     int64_t launches = 0;
     std::string msg;
 
@@ -596,9 +596,8 @@ struct pdlpgpu_mlp {
                            const Gradients& g) {
         AdamStep adam{lr, 0.9f, 0.999f, 1e-8f, 1.0f, 1.0f, 1.0f, 1.0f};
         if (train) {
-            ++step;
-            adam.c1 = 1.0f - std::pow(adam.b1, static_cast<float>(step));
-            adam.c2 = 1.0f - std::pow(adam.b2, static_cast<float>(step));
+            adam.c1 = 1.0f - std::pow(adam.b1, static_cast<float>(step + 1));
+            adam.c2 = 1.0f - std::pow(adam.b2, static_cast<float>(step + 1));
             adam.r1 = 1.0f / adam.c1;
             adam.r2 = 1.0f / adam.c2;
         }
@@ -647,6 +646,7 @@ struct pdlpgpu_mlp {
             msg = "Adam launch failed";
             return false;
         }
+        ++step;   // a refused call does not count
         return true;
     }
 
