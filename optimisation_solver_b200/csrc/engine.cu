@@ -1009,22 +1009,27 @@ void Engine::choose_fused() {
     fused_cluster_ = cluster;
 }
 
-void Engine::enqueue_chunk(int slots, bool fp64_stage) {
+bool Engine::enqueue_chunk(int slots, bool fp64_stage) {
     if (fused_cluster_ > 0) {
         // One launch runs every instance's trials of the interval.
         const int V = tuning_.vector_width;
+        auto fused64 = [&] {
+            return launch_fused<double>(g_, w64_, dopt_, V, count_, fused_cluster_, slots, fused_shape64_, stream_);
+        };
         record_timing(0);
-        if (mixed_) launch_fused<float>(g_, w32_, dopt_, V, count_, fused_cluster_, slots, fused_shape32_, stream_);
-        else launch_fused<double>(g_, w64_, dopt_, V, count_, fused_cluster_, slots, fused_shape64_, stream_);
+        if (!check(mixed_ ? launch_fused<float>(g_, w32_, dopt_, V, count_, fused_cluster_, slots, fused_shape32_,
+                                                stream_)
+                          : fused64(), "fused trials"))
+            return false;
         launches_ += 1;
         if (mixed_ && fp64_stage) {
-            launch_fused<double>(g_, w64_, dopt_, V, count_, fused_cluster_, slots, fused_shape64_, stream_);
+            if (!check(fused64(), "fused trials")) return false;
             launches_ += 1;
         }
         record_timing(1);
         enqueue_check_stage(true);
         record_timing(2);
-        return;
+        return true;
     }
     // A mixed solve iterates in FP32; while some instance is in its FP64
     // stage, each slot also launches the per-instance FP64 trial kernels
@@ -1060,6 +1065,7 @@ void Engine::enqueue_chunk(int slots, bool fp64_stage) {
     record_timing(1);
     enqueue_check_stage(true);
     record_timing(2);
+    return true;
 }
 
 void Engine::timing_reset() {
@@ -1120,9 +1126,14 @@ bool Engine::build_graph(int slots, bool fp64_stage) {
     if (!check(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture"))
         return false;
     const int64_t before = launches_;
-    enqueue_chunk(slots, fp64_stage);
+    const bool enqueued = enqueue_chunk(slots, fp64_stage);
     launches_ = before;
-    if (!check(cudaStreamEndCapture(stream_, &graph), "end capture")) return false;
+    const cudaError_t ended = cudaStreamEndCapture(stream_, &graph);
+    if (!enqueued || !check(ended, "end capture")) {
+        if (graph != nullptr) cudaGraphDestroy(graph);
+        cudaGetLastError();   // reported here, not by the thread's next solve
+        return false;
+    }
     const bool ok = check(cudaGraphInstantiate(fp64_stage ? &graph64_ : &graph_, graph, 0), "graph instantiate");
     cudaGraphDestroy(graph);
     graph_slots_ = slots;
@@ -1136,8 +1147,7 @@ bool Engine::launch_chunk(int slots) {
     const int trial_launches = fused_cluster_ > 0 ? (fp64 ? 2 : 1) : (il_ ? 2 : 3) * slots * (fp64 ? 2 : 1);
     const int per_chunk = trial_launches + check_stage_launches(true);
     if (spec_.ext.disable_graphs) {
-        enqueue_chunk(slots, fp64);
-        return check(cudaGetLastError(), "chunk launch");
+        return enqueue_chunk(slots, fp64) && check(cudaGetLastError(), "chunk launch");
     }
     cudaGraphExec_t& g = fp64 ? graph64_ : graph_;
     if (g == nullptr && !build_graph(slots, fp64)) return false;

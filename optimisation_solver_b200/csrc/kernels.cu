@@ -1982,8 +1982,13 @@ bool fused_config(K kernel, int count, int cluster, const FusedShape& shape, cud
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    // Clusters of 16 CTAs are beyond the portable size of 8.
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+    // The limit is the kernel's, shared by every engine of the process, so all
+    // set the same one: an engine that set its own size would lower it between
+    // another's query and its launch. Clusters of 16 CTAs are beyond the
+    // portable size of 8.
+    static_assert(kFusedMaxSmemHost + sizeof(FusedCta) <= 227 * 1024, "beside the static shared memory");
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kFusedMaxSmemHost)) == cudaSuccess &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
         return true;
     cudaGetLastError();
