@@ -29,6 +29,8 @@
 
 #include <cstdint>
 
+#include "team_walk.hpp"
+
 namespace pdlpgpu_mlp_impl {
 
 using bf16 = __nv_bfloat16;
@@ -808,66 +810,69 @@ __global__ void __launch_bounds__(kAdamThreads, 1) adam_step(const __grid_consta
         // The biases' warps sit in the last CTAs, which have the fewest tiles.
         const int job = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * 8 * kAdamTeams + (warp - 4);
         for (int b = job; b < bias_warps(a.bias.H); b += 8 * kAdamTeams * step) bias_and_loss_warp(a.bias, b);
-        int n = 0, k = 0, mine = 0;   // chunks and tiles of the CTA, chunks of the team
-        for (int t = blockIdx.x; t < a.tiles && good; t += step, ++k) {
-            int m0, n0;
-            const AdamLayer& L = locate(t, m0, n0);
-            const int q = k & 1;
-            good = mbar_wait(smem_u32(&acc_full[q]), (k / 2) & 1, a.err, 4);
-            for (int c = 0; c < kAdamBN && n0 + c < L.cols; c += 32, ++n) {
-                if (n % kAdamTeams != team) continue;
-                good = mbar_wait(smem_u32(&slot_full[team]), mine++ & 1, a.err, 7) && good;
-                good = all_good(good, 1 + team);
-                if (!good) break;
-                tc_fence_after();
-                uint32_t g[16];
-                tmem_ld16(tmem + (static_cast<uint32_t>(quad * 32) << 16) + q * kAdamBN + c + 16 * part, g);
-                uint32_t h[8];
+        int m0 = 0, n0 = 0;
+        const AdamLayer* L = nullptr;
+        auto chunks = [&](int t) {
+            L = &locate(t, m0, n0);
+            return min(kAdamBN, L->cols - n0 + 31) / 32;
+        };
+        auto wait_tile = [&](int k) { return mbar_wait(smem_u32(&acc_full[k & 1]), (k / 2) & 1, a.err, 4); };
+        auto wait_chunk = [&](int i) { return mbar_wait(smem_u32(&slot_full[team]), i & 1, a.err, 7); };
+        auto agree = [&](bool ok) { return all_good(ok, 1 + team); };
+        auto work = [&](int k, int chunk) {
+            const int q = k & 1, c = 32 * chunk;
+            tc_fence_after();
+            uint32_t g[16];
+            tmem_ld16(tmem + (static_cast<uint32_t>(quad * 32) << 16) + q * kAdamBN + c + 16 * part, g);
+            uint32_t h[8];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int off = row * 128 + (((4 * part + j) ^ (row & 7)) << 4);
-                    float4* pp = reinterpret_cast<float4*>(at + off);
-                    float4* pm = reinterpret_cast<float4*>(at + kChunkBytes + off);
-                    float4* pv = reinterpret_cast<float4*>(at + 2 * kChunkBytes + off);
-                    float4 p = *pp, m = *pm, v = *pv;
-                    const float gj[4] = {__uint_as_float(g[4 * j]), __uint_as_float(g[4 * j + 1]),
-                                         __uint_as_float(g[4 * j + 2]), __uint_as_float(g[4 * j + 3])};
-                    a.adam(gj, p, m, v);
-                    *pp = p;
-                    *pm = m;
-                    *pv = v;
-                    h[2 * j] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.x))) |
-                               (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.y))) << 16);
-                    h[2 * j + 1] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.z))) |
-                                   (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.w))) << 16);
-                }
-                uint8_t* ph = at + 3 * kChunkBytes + row * 64;
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    *reinterpret_cast<uint4*>(ph + (((2 * part + j) ^ ((row >> 1) & 3)) << 4)) =
-                        make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
-                // The chunk goes out as the eight warps leave it, and the
-                // slot is free once the store has read it.
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                asm volatile("bar.sync %0, 256;" ::"r"(1 + kAdamTeams + team) : "memory");
-                if (quad == 0 && part == 0 && lane == 0) {
-                    const uint32_t src = smem_u32(at);
-                    tma_store_2d(&L.p, src, n0 + c, m0);
-                    tma_store_2d(&L.m, src + kChunkBytes, n0 + c, m0);
-                    tma_store_2d(&L.v, src + 2 * kChunkBytes, n0 + c, m0);
-                    tma_store_2d(&L.h, src + 3 * kChunkBytes, n0 + c, m0);
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    mbar_arrive(smem_u32(&slot_empty[team]));
-                }
-                __syncwarp();
+            for (int j = 0; j < 4; ++j) {
+                const int off = row * 128 + (((4 * part + j) ^ (row & 7)) << 4);
+                float4* pp = reinterpret_cast<float4*>(at + off);
+                float4* pm = reinterpret_cast<float4*>(at + kChunkBytes + off);
+                float4* pv = reinterpret_cast<float4*>(at + 2 * kChunkBytes + off);
+                float4 p = *pp, m = *pm, v = *pv;
+                const float gj[4] = {__uint_as_float(g[4 * j]), __uint_as_float(g[4 * j + 1]),
+                                     __uint_as_float(g[4 * j + 2]), __uint_as_float(g[4 * j + 3])};
+                a.adam(gj, p, m, v);
+                *pp = p;
+                *pm = m;
+                *pv = v;
+                h[2 * j] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.x))) |
+                           (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.y))) << 16);
+                h[2 * j + 1] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.z))) |
+                               (static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(p.w))) << 16);
             }
-            // Every team is done with the tile's accumulator.
+            uint8_t* ph = at + 3 * kChunkBytes + row * 64;
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                *reinterpret_cast<uint4*>(ph + (((2 * part + j) ^ ((row >> 1) & 3)) << 4)) =
+                    make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
+            // The chunk goes out as the eight warps leave it, and the
+            // slot is free once the store has read it.
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            asm volatile("bar.sync %0, 256;" ::"r"(1 + kAdamTeams + team) : "memory");
+            if (quad == 0 && part == 0 && lane == 0) {
+                const uint32_t src = smem_u32(at);
+                tma_store_2d(&L->p, src, n0 + c, m0);
+                tma_store_2d(&L->m, src + kChunkBytes, n0 + c, m0);
+                tma_store_2d(&L->v, src + 2 * kChunkBytes, n0 + c, m0);
+                tma_store_2d(&L->h, src + 3 * kChunkBytes, n0 + c, m0);
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                mbar_arrive(smem_u32(&slot_empty[team]));
+            }
+            __syncwarp();
+        };
+        // Every team is done with the tile's accumulator.
+        auto leave = [&](int k) {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[q]));
-        }
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[k & 1]));
+        };
+        good = team_walk(static_cast<int>(blockIdx.x), step, a.tiles, team, kAdamTeams, chunks, wait_tile, wait_chunk,
+                         agree, work, leave);
         if (quad == 0 && part == 0 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     if (!good) drain_pause();
