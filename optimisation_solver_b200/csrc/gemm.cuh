@@ -10,7 +10,6 @@
 //               into the loss, its gradient and the bias update
 //   adam_step   the weight gradients of a training step, each tile straight
 //               into its weights' Adam step
-//   gemm_split  few tiles and a long K: the splits of a tile in a cluster
 //   gemm_pair   large plain products: two CTAs share a 256 x 256 tile
 //               (cta_group::2), persistent, the epilogue of one tile under
 //               the main loop of the next
@@ -883,174 +882,6 @@ __global__ void __launch_bounds__(kAdamThreads, 1) adam_step(const __grid_consta
 }
 
 // ---------------------------------------------------------------------------
-// gemm_split: few output tiles and a long K: the CTAs of a cluster run the
-// splits of one 128 x 128 tile side by side and add them through distributed
-// shared memory, in split order -- no scratch in device memory and no second
-// kernel. Each CTA holds up to four splits' accumulators in TMEM.
-// ---------------------------------------------------------------------------
-constexpr int kSplitStages = 6;
-constexpr int kSplitAccs = 4;
-constexpr int kSplitRanks = 8;   // a cluster at most
-constexpr int kSplitSmem = tile_smem<128, kSplitStages>();
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-
-__global__ void __launch_bounds__(kTileThreads, 1)
-gemm_split(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TileArgs a,
-           int log_ranks, float* C) {
-    constexpr uint32_t kBytes = BM * BK * 2;   // of either operand
-    constexpr uint32_t kIdesc = instr_desc(BM, 128, false, false);
-    constexpr int S = kSplitStages;
-    static_assert(S * 2 * kBytes >= 2 * BM * 129 * 4 && S * 2 * kBytes >= kSplitAccs * BM * 65 * 4,
-                  "the drained ring holds a slab of every split");
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = align1024(smem_raw);
-    uint8_t* sa = smem;
-    uint8_t* sb = smem + S * kBytes;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sb + S * kBytes);
-    uint64_t *full = bars, *empty = bars + S, *done = bars + 2 * S;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 1);
-    __shared__ int consumed_by_mma;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = static_cast<int>(cluster_rank());   // along x
-    const int ranks = 1 << log_ranks;
-    const int tile = static_cast<int>(blockIdx.x) >> log_ranks, tiles_m = (a.M + BM - 1) / BM;
-    const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * 128;
-    const int total_kb = (a.K + BK - 1) / BK;
-    // Splits [z0, z1) of rank r: as even as whole splits allow.
-    auto first = [&](int r) { return (r * a.splits) >> log_ranks; };
-    const int z0 = first(rank), z1 = first(rank + 1);
-    const int kb0 = min(total_kb, z0 * a.kb_per_split);
-    const int nk = min(total_kb, z1 * a.kb_per_split) - kb0;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < S; ++s) {
-            mbar_init(smem_u32(&full[s]), 1);
-            mbar_init(smem_u32(&empty[s]), 1);
-        }
-        mbar_init(smem_u32(done), 1);
-        consumed_by_mma = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (warp == 0) tmem_alloc(smem_u32(tmem_slot), 512);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
-    int issued = 0;
-    Ring<S> ring;
-    if (warp == 0) {
-        for (int i = 0; i < nk; ++i, ring.next()) {
-            const int s = ring.s;
-            if (ring.wrapped && !warp_wait(smem_u32(&empty[s]), ring.phase ^ 1, a.err, 2)) break;
-            if (elect_one()) {
-                const uint32_t fb = smem_u32(&full[s]);
-                mbar_expect_tx(fb, 2 * kBytes);
-                load_operand<false, BM>(smem_u32(sa + s * kBytes), &map_a, fb, kb0 + i, m0);
-                load_operand<false, 128>(smem_u32(sb + s * kBytes), &map_b, fb, kb0 + i, n0);
-            }
-            ++issued;
-        }
-    } else if (warp == 1) {
-        int i = 0, left = a.kb_per_split;
-        uint32_t acc = tmem, more = 0;
-        for (; i < nk; ++i, ring.next()) {
-            const int s = ring.s;
-            if (!warp_wait(smem_u32(&full[s]), ring.phase, a.err, 1)) break;
-            tc_fence_after();
-            const uint64_t da = smem_desc<false>(smem_u32(sa + s * kBytes));
-            const uint64_t db = smem_desc<false>(smem_u32(sb + s * kBytes));
-            if (elect_one()) {
-#pragma unroll
-                for (int kk = 0; kk < BK / 16; ++kk) mma_bf16(acc, da + kk * 2, db + kk * 2, kIdesc, kk > 0 ? 1u : more);
-                mma_commit(smem_u32(&empty[s]));
-            }
-            more = 1;
-            if (--left == 0) {
-                left = a.kb_per_split;
-                acc += 128;
-                more = 0;
-            }
-        }
-        if (elect_one()) {
-            consumed_by_mma = i;
-            mma_commit(smem_u32(done));
-        }
-        __syncwarp();
-    }
-    __syncthreads();
-    if (warp == 0 && lane == 0)
-        for (int i = consumed_by_mma; i < issued; ++i)
-            mbar_wait(smem_u32(&full[i % S]), (i / S) & 1, a.err, 3);
-    const bool have = mbar_wait(smem_u32(done), 0, a.err, 4);
-    __syncthreads();
-    tc_fence_after();
-
-    // Every CTA puts its splits' values in shared memory (all 128 columns at
-    // once where two splits a CTA leave room, else 64), then CTA r adds rows
-    // r * 128 / ranks .. of all of them: every rank's values of a row piece
-    // are on their way before the first is added.
-    float* slab = reinterpret_cast<float*>(sa);   // [splits of the CTA][128][width + 1]
-    const int most = (a.splits + ranks - 1) >> log_ranks;
-    const int width = most <= 2 ? 128 : 64, pitch = width + 1;
-    const int rows = BM >> log_ranks, pieces = width / 32;
-    for (int w0 = 0; w0 < 128; w0 += width) {
-        const int row = (warp & 3) * 32 + lane;
-        for (int job = warp >> 2; job < (z1 - z0) * pieces; job += 2) {
-            const int q = job / pieces, c = (job - q * pieces) * 32;
-            uint32_t r[32];
-            tmem_ld32(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + q * 128 + w0 + c, r);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) slab[(q * BM + row) * pitch + c + j] = have ? __uint_as_float(r[j]) : 0.0f;
-        }
-        cluster_sync();
-        for (int job = warp; job < rows * pieces; job += kTileThreads / 32) {
-            const int rr = job / pieces, c = (job - rr * pieces) * 32 + lane;
-            const int line = rank * rows + rr;
-            float v[kSplitRanks][kSplitAccs];
-            const uint32_t at = smem_u32(slab + line * pitch + c);
-#pragma unroll
-            for (int r = 0; r < kSplitRanks; ++r) {
-                const int count = r < ranks ? first(r + 1) - first(r) : 0;
-                const uint32_t there = map_rank(at, static_cast<uint32_t>(r < ranks ? r : 0));
-#pragma unroll
-                for (int q = 0; q < kSplitAccs; ++q)
-                    if (q < count)
-                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[r][q]) : "r"(there + q * BM * pitch * 4));
-            }
-            float sum = 0.0f;
-#pragma unroll
-            for (int r = 0; r < kSplitRanks; ++r) {
-                const int count = r < ranks ? first(r + 1) - first(r) : 0;
-#pragma unroll
-                for (int q = 0; q < kSplitAccs; ++q)
-                    if (q < count) sum += v[r][q];
-            }
-            const int col = n0 + w0 + c;
-            if (m0 + line < a.M && col < a.N) C[static_cast<int64_t>(m0 + line) * a.N + col] = sum;
-        }
-        cluster_sync();
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_free(tmem, 512);
-}
-
-// ---------------------------------------------------------------------------
 // last_layer: out = H W^T + bias over one tile of `bn` columns and all rows,
 // 128 at a time. A forward pass stores it; a training step goes on to
 //   e = out - target,  loss += w e^2,
@@ -1364,6 +1195,21 @@ struct PairArgs {
     float* C;
     int* err;
 };
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
 
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int32_t x,
                                                  int32_t y) {

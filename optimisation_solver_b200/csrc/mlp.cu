@@ -100,6 +100,34 @@ __global__ void __launch_bounds__(32) bias_and_loss(BiasArgs a) {
     bias_and_loss_warp(a, static_cast<int>(blockIdx.x));
 }
 
+// C = the splits' partials added in split order, four neighbouring elements a
+// thread where C allows 16-byte stores, else one. Sixteen splits' loads are in
+// flight before the first is added.
+template <int kPer>
+__global__ void __launch_bounds__(128) add_splits(const float* partial, int splits, int64_t total, float* C) {
+    pdl_trigger();
+    pdl_wait();
+    const int64_t t = kPer * (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x);
+    if (t >= total) return;
+    if constexpr (kPer == 4) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 16
+        for (int z = 0; z < splits; ++z) {
+            const float4 p = *reinterpret_cast<const float4*>(partial + z * total + t);
+            v.x += p.x;
+            v.y += p.y;
+            v.z += p.z;
+            v.w += p.w;
+        }
+        *reinterpret_cast<float4*>(C + t) = v;
+    } else {
+        float v = 0.0f;
+#pragma unroll 16
+        for (int z = 0; z < splits; ++z) v += partial[z * total + t];
+        C[t] = v;
+    }
+}
+
 __global__ void to_bf16(const float* src, bf16* dst, int64_t n) {
     for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n;
          t += static_cast<int64_t>(gridDim.x) * blockDim.x)
@@ -315,78 +343,15 @@ bool tile_gemm(const bf16* A, const bf16* B, int M, int N, int K, Splits sp, boo
     return true;
 }
 
-// C = A B^T for the two entry points below, without scratch in device memory.
-// The rule, with times in us of the kernels that meet at each line:
-//   one split, at least 56 tiles of 256 x 256 and 1792 tile x K-block steps:
-//     gemm_pair (4096 x 2048 x 4096: 51, gemm_tile 63; 2048^3 21, 21;
-//     4096 x 2048 x 512, below the line: 21 against 19)
-//   several splits on few 128 x 128 tiles: gemm_split, as long as a tile's
-//     CTA would otherwise run long alone (600 x 600 x 8000 in 8 splits: 43 in
-//     one CTA a tile; 300 x 2000 x 8000 in 3, above the line: 35)
-//   else gemm_tile, each CTA its tile's splits in turn: six stages and an SM
-//     to itself while the tiles fit the SMs once or a tile has several splits
-//     to keep apart in TMEM (3000 x 2000 x 4096 in 8: 88, with three stages
-//     184), else three stages and two CTAs an SM (2560 x 1024 x 1024, 160
-//     tiles: 14, with six 19).
-constexpr int64_t kPairMinTiles = 56;
-constexpr int64_t kPairMinSteps = 1792;
-constexpr int64_t kSplitMaxTiles = 40;
-
-bool plain_gemm(const bf16* A, const bf16* B, float* C, int M, int N, int K, int splits, int* err, cudaStream_t s,
-                std::string& msg) {
-    if (K % 8 != 0) {
-        msg = "GEMM K must be a multiple of 8";
-        return false;
-    }
-    const Splits sp = effective_splits(K, splits);
-    const int64_t pair_tiles = int64_t((M + 255) / 256) * ((N + 255) / 256);
-    const int64_t tiles = int64_t((M + BM - 1) / BM) * ((N + 127) / 128);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sp.count == 1 && pair_tiles >= kPairMinTiles && pair_tiles * ((K + BK - 1) / BK) >= kPairMinSteps) {
-        static bool smem_set[64] = {false};
-        if (!allow_smem(reinterpret_cast<const void*>(gemm_pair), kPairSmem, smem_set, msg)) return false;
-        CUtensorMap ma, mb;
-        if (!make_map(ma, A, M, K, BK, BM, msg) || !make_map(mb, B, N, K, BK, BM, msg)) return false;
-        const PairArgs pa{M, N, K, C, err};
-        const unsigned pairs = static_cast<unsigned>(std::min<int64_t>(pair_tiles, sms / 2));
-        return launch(gemm_pair, dim3(2 * pairs), kPairThreads, kPairSmem, s, false, 1, ma, mb, pa);
-    }
-    if (sp.count > 1 && sp.count <= kSplitRanks * kSplitAccs && tiles < kSplitMaxTiles) {
-        static bool smem_set[64] = {false};
-        if (!allow_smem(reinterpret_cast<const void*>(gemm_split), kSplitSmem, smem_set, msg)) return false;
-        CUtensorMap ma, mb;
-        if (!make_map(ma, A, M, K, BK, BM, msg) || !make_map(mb, B, N, K, BK, 128, msg)) return false;
-        // The cluster: as many of the splits side by side as the SMs hold,
-        // and no more accumulators in a CTA than TMEM does.
-        int log_ranks = 1;
-        while ((1 << log_ranks) < kSplitRanks && (2 << log_ranks) <= sp.count &&
-               ((2 * tiles) << log_ranks) <= sms)
-            ++log_ranks;
-        while ((kSplitAccs << log_ranks) < sp.count) ++log_ranks;
-        const TileArgs ta{M, N, K, sp.per, sp.count, err};
-        return launch(gemm_split, dim3(static_cast<unsigned>(tiles << log_ranks)), kTileThreads, kSplitSmem, s, false,
-                      1 << log_ranks, ma, mb, ta, log_ranks, C);
-    }
-    const EpiStore epi{C, 0, nullptr};
-    if (tiles <= sms || sp.count > 1)
-        return tile_gemm<128, 6, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
-    return tile_gemm<128, 3, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
-}
-
-int splits_for(int M, int N, int K) {
-    const int tiles = ((M + BM - 1) / BM) * ((N + 127) / 128);
-    const int kb = (K + BK - 1) / BK;
-    int s = std::max(1, 148 / std::max(1, tiles));
-    return std::min(s, std::max(1, kb / 4));
-}
-
 // Error words of calls that have no model to keep one: a slot of this
 // static array per call in flight, so calls of several threads do not see
 // one another's errors. A slot is zero whenever it is free.
 constexpr int kErrSlots = 64;
 __device__ int g_gemm_err[kErrSlots];
+// The partials of a call's K splits, M x N of every split (74 tiles in 16 splits:
+// 78 MB): static, so that no call allocates, and of the call that holds slot 0.
+constexpr int64_t kScratchTiles = 1184;   // of 128 x 128
+__device__ float4 g_gemm_scratch[kScratchTiles * BM * 128 / 4];
 std::mutex g_err_mutex;
 uint64_t g_err_used = 0;
 
@@ -412,6 +377,12 @@ struct ErrSlot {
             cudaMemset(address, 0, sizeof(int));
         }
     }
+    // The scratch for partials, where this call holds it.
+    float* scratch() const {
+        void* base = nullptr;
+        return slot == 0 && cudaGetSymbolAddress(&base, g_gemm_scratch) == cudaSuccess ? static_cast<float*>(base)
+                                                                                       : nullptr;
+    }
     // Waits for the default stream and returns the error word, clearing it;
     // a negative value is a CUDA error.
     int take() {
@@ -430,6 +401,75 @@ struct ErrSlot {
     ErrSlot(const ErrSlot&) = delete;
     ErrSlot& operator=(const ErrSlot&) = delete;
 };
+
+// C = A B^T for the two entry points below. The rule, with times in us of the
+// kernels that meet at each line:
+//   one split, at least 56 tiles of 256 x 256 and 1792 tile x K-block steps:
+//     gemm_pair (4096 x 2048 x 4096: 51, gemm_tile 63; 2048^3 21, 21;
+//     4096 x 2048 x 512, below the line: 21 against 19)
+//   several splits: gemm_tile with a CTA for every split of every tile, the
+//     partials in `scratch` and added by add_splits, as long as the splits make
+//     up for the waves of CTAs (K = 8000, in brackets each CTA its tile's splits
+//     in turn: 60 tiles in 8 splits 30 [47], in 16 49 [72], 96 in 3 29 [35], in 12
+//     59 [60]; beyond the line 104 in 8 50 [48], 147 in 2 41 [37]; 256 x 512 x
+//     22000 in 18 takes 16). Six stages and an SM to itself while the CTAs fit the SMs once, else
+//     three and two CTAs an SM (24 tiles in 8: 17, with six 22). The clusters of
+//     CTAs that added their splits through distributed shared memory took 33 at
+//     256 x 512 x 22000, 27 with wide loads, and 51 and 25 for two splits of one
+//     tile (23 this way).
+//   else gemm_tile, each CTA its tile's splits in turn: six stages and an SM
+//     to itself while the tiles fit the SMs once or a tile has several splits
+//     to keep apart in TMEM (3000 x 2000 x 4096 in 8: 88, with three stages
+//     184), else three stages and two CTAs an SM (2560 x 1024 x 1024, 160
+//     tiles: 14, with six 19).
+constexpr int64_t kPairMinTiles = 56;
+constexpr int64_t kPairMinSteps = 1792;
+
+bool plain_gemm(const bf16* A, const bf16* B, float* C, int M, int N, int K, int splits, float* scratch, int* err,
+                cudaStream_t s, std::string& msg) {
+    if (K % 8 != 0) {
+        msg = "GEMM K must be a multiple of 8";
+        return false;
+    }
+    const Splits sp = effective_splits(K, splits);
+    const int64_t pair_tiles = int64_t((M + 255) / 256) * ((N + 255) / 256);
+    const int64_t tiles = int64_t((M + BM - 1) / BM) * ((N + 127) / 128);
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sp.count == 1 && pair_tiles >= kPairMinTiles && pair_tiles * ((K + BK - 1) / BK) >= kPairMinSteps) {
+        static bool smem_set[64] = {false};
+        if (!allow_smem(reinterpret_cast<const void*>(gemm_pair), kPairSmem, smem_set, msg)) return false;
+        CUtensorMap ma, mb;
+        if (!make_map(ma, A, M, K, BK, BM, msg) || !make_map(mb, B, N, K, BK, BM, msg)) return false;
+        const PairArgs pa{M, N, K, C, err};
+        const unsigned pairs = static_cast<unsigned>(std::min<int64_t>(pair_tiles, sms / 2));
+        return launch(gemm_pair, dim3(2 * pairs), kPairThreads, kPairSmem, s, false, 1, ma, mb, pa);
+    }
+    const int64_t ctas = tiles * sp.count, waves = (ctas + 2 * sms - 1) / (2 * sms);
+    if (sp.count > 1 && scratch != nullptr && ctas <= kScratchTiles && (ctas <= sms || 3 * waves <= sp.count)) {
+        const int64_t total = int64_t(M) * N;
+        const EpiStore epi{scratch, total, nullptr};
+        if (!(ctas <= sms ? tile_gemm<128, 6, false, false>(A, B, M, N, K, sp, true, epi, err, s, false, msg)
+                          : tile_gemm<128, 3, false, false>(A, B, M, N, K, sp, true, epi, err, s, false, msg)))
+            return false;
+        const bool wide = total % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+        const int64_t threads = wide ? total / 4 : total;
+        return launch(wide ? add_splits<4> : add_splits<1>, dim3(static_cast<unsigned>((threads + 127) / 128)), 128, 0, s,
+                      true, 1, scratch, sp.count, total, C);
+    }
+    const EpiStore epi{C, 0, nullptr};
+    if (tiles <= sms || sp.count > 1)
+        return tile_gemm<128, 6, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
+    return tile_gemm<128, 3, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
+}
+
+int splits_for(int M, int N, int K) {
+    const int tiles = ((M + BM - 1) / BM) * ((N + 127) / 128);
+    const int kb = (K + BK - 1) / BK;
+    int s = std::max(1, 148 / std::max(1, tiles));
+    return std::min(s, std::max(1, kb / 4));
+}
 
 }  // namespace pdlpgpu_mlp_impl
 
@@ -818,7 +858,7 @@ int32_t pdlpgpu_gemm_bf16(int32_t M, int32_t N, int32_t K, const uint16_t* A, co
     if (err.address == nullptr) return fail("gemm: no error word");
     std::string msg;
     bool ok = plain_gemm(reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(B), C, M, N, K, splits,
-                         err.address, nullptr, msg);
+                         err.scratch(), err.address, nullptr, msg);
     const int h = err.take();
     if (h > 0) msg = "tensor-core pipeline wait timed out (code " + std::to_string(h) + ")";
     ok = ok && h == 0;
@@ -835,7 +875,7 @@ int32_t pdlpgpu_gemm_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, co
     std::string msg;
     auto once = [&]() {
         return plain_gemm(reinterpret_cast<const bf16*>(A), reinterpret_cast<const bf16*>(B), C, M, N, K, splits,
-                          err.address, nullptr, msg);
+                          err.scratch(), err.address, nullptr, msg);
     };
     bool ok = once();   // warm-up: tensor maps, instruction cache
     cudaEvent_t e0, e1;
