@@ -894,6 +894,9 @@ __global__ void __launch_bounds__(kAdamThreads, 1) adam_step(const __grid_consta
 // Warp 0 loads, warp 1 multiplies (two sets of accumulators while TMEM has
 // room, so a row tile's products run under the previous one's epilogue);
 // two teams of four epilogue warps take the 32-column blocks in turn.
+// In a forward pass the row tiles may be dealt over gridDim.y CTAs (a batch of
+// many rows and few columns); a training step adds the bias gradient over all
+// rows in order and has one.
 // ---------------------------------------------------------------------------
 struct LastArgs {
     int M, N, K, bn;
@@ -964,7 +967,7 @@ last_layer(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     if (warp == 0) {
         Ring<S> ring;
         bool good = true;
-        for (int mt = 0; mt < mts && good; ++mt)
+        for (int mt = blockIdx.y; mt < mts && good; mt += gridDim.y)
             for (int kb = 0; kb < kbs; ++kb, ring.next()) {
                 const int s = ring.s;
                 if (ring.wrapped && !warp_wait(smem_u32(&empty[s]), ring.phase ^ 1, a.err, 2)) {
@@ -983,9 +986,9 @@ last_layer(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         int i = 0;
         Ring<S> ring;
         bool good = true;
-        for (int mt = 0; mt < mts && good; ++mt) {
-            const int q = sets == 2 ? mt & 1 : 0;
-            if (mt >= sets && !warp_wait(smem_u32(&acc_empty[q]), ((sets == 2 ? mt >> 1 : mt) - 1) & 1, a.err, 5)) break;
+        for (int mt = blockIdx.y, t = 0; mt < mts && good; mt += gridDim.y, ++t) {
+            const int q = sets == 2 ? t & 1 : 0;
+            if (t >= sets && !warp_wait(smem_u32(&acc_empty[q]), ((sets == 2 ? t >> 1 : t) - 1) & 1, a.err, 5)) break;
             tc_fence_after();
             uint32_t acc = tmem + static_cast<uint32_t>(q * a.splits * a.bn), more = 0;
             int left = a.kb_per_split;
@@ -1045,9 +1048,9 @@ last_layer(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             }
         };
         if (team < blocks) load_targets(0, team);
-        for (int mt = 0; mt < mts; ++mt) {
-            const int m0 = mt * BM, q = sets == 2 ? mt & 1 : 0;
-            const bool have = mbar_wait(smem_u32(&acc_full[q]), (sets == 2 ? mt >> 1 : mt) & 1, a.err, 4);
+        for (int mt = blockIdx.y, u = 0; mt < mts; mt += gridDim.y, ++u) {
+            const int m0 = mt * BM, q = sets == 2 ? u & 1 : 0;
+            const bool have = mbar_wait(smem_u32(&acc_full[q]), (sets == 2 ? u >> 1 : u) & 1, a.err, 4);
             tc_fence_after();
             __syncwarp();
             for (int b = team; b < blocks; b += 2) {

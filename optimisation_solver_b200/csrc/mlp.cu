@@ -560,7 +560,9 @@ struct pdlpgpu_mlp {
     bool hidden_product(const bf16* A, const bf16* B, int K, Splits& sp) {
         sp = effective_splits(K, splits_for(batch, hidden, K));
         const EpiStore epi{partial, int64_t(batch) * hidden, nullptr};
-        return product<6, false, kBMn>(A, B, batch, hidden, K, sp, epi);
+        const int64_t ctas = int64_t((batch + BM - 1) / BM) * ((hidden + 127) / 128) * sp.count;
+        return ctas <= sms ? product<6, false, kBMn>(A, B, batch, hidden, K, sp, epi)
+                           : product<3, false, kBMn>(A, B, batch, hidden, K, sp, epi);
     }
 
     int hidden_ctas() const { return static_cast<int>((int64_t(batch) * hidden / 4 + 127) / 128); }
@@ -579,10 +581,30 @@ struct pdlpgpu_mlp {
     int last_bn() const { return std::min(256, ((out + sms - 1) / sms + 31) / 32 * 32); }
     int last_ctas() const { return (out + last_bn() - 1) / last_bn(); }
 
+    // A forward pass of a batch of many rows may share the row tiles of wider
+    // column tiles instead. What counts is the bytes a CTA copies into shared
+    // memory, 128 + bn rows of both operands per K block and row tile
+    // (a forward pass of 1024 x 512 x 64, batch 8192: 69 us, 203 with two CTAs; 2048 x
+    // 1024 x 2048, batch 4096: 94 and 205). The K splits, and with them the
+    // bits, stay.
+    void forward_tile(int splits, int& bn, int& rows) const {
+        const int mts = (batch + BM - 1) / BM;
+        int64_t least = INT64_MAX;
+        for (int n = last_bn(); n <= 256 && n * splits <= kLastTmem; n += 32) {
+            const int ctas = (out + n - 1) / n, share = std::max(1, std::min(mts, sms / ctas));
+            const int64_t cost = int64_t((mts + share - 1) / share) * (BM + n) * ((ctas * share + sms - 1) / sms);
+            if (cost >= least) continue;
+            least = cost;
+            bn = n;
+            rows = share;
+        }
+    }
+
     template <bool kTrain>
     bool last(LastArgs la) {
-        const int bn = last_bn();
+        int bn = last_bn(), rows = 1;   // CTAs that share the batch's row tiles
         const Splits sp = effective_splits(hidden, std::min(splits_for(batch, out, hidden), kLastTmem / bn));
+        if (!kTrain) forward_tile(sp.count, bn, rows);
         la.M = batch;
         la.N = out;
         la.K = hidden;
@@ -596,8 +618,8 @@ struct pdlpgpu_mlp {
         CUtensorMap ma, mb;
         if (!make_map(ma, H2, batch, hidden, BK, BM, msg) || !make_map(mb, W3h, out, hidden, BK, bn, msg)) return false;
         ++launches;
-        if (launch(last_layer<kTrain>, dim3(static_cast<unsigned>(last_ctas())), kLastThreads, last_smem(bn), stream, true,
-                   1, ma, mb, la))
+        if (launch(last_layer<kTrain>, dim3(static_cast<unsigned>((out + bn - 1) / bn), static_cast<unsigned>(rows)),
+                   kLastThreads, last_smem(bn), stream, true, 1, ma, mb, la))
             return true;
         msg = "GEMM launch failed";
         return false;
