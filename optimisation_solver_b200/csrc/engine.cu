@@ -931,6 +931,7 @@ void Engine::choose_fused() {
     auto last = [](const std::vector<CtaWork>& side, int e1) { return side[static_cast<size_t>(e1 - 1)].slice_end; };
     FusedShape sh{};
     sh.elem = static_cast<int32_t>(sizeof(double));
+    sh.limits = dopt_.time_limit > 0.0 || !dopt_.adaptive;
     int32_t rows = 0, cols_rows = 0;   // most 2 m and 2 m + n of an instance
     for (int b = 0; b < count_; ++b) {
         const InstanceInfo& inf = info_[static_cast<size_t>(b)];

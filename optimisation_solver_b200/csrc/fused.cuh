@@ -16,8 +16,11 @@
 // k_dual's fixed order, so an instance's results are the two-kernel path's
 // bit for bit; every CTA adds the same numbers, so all of them agree without
 // being told. What that does not cover -- the check boundary, limits, a
-// clock, non-finite sums -- goes through trial_control in rank 0, whose
-// control block is then copied to the others.
+// clock that has run out, non-finite sums -- goes through trial_control in rank
+// 0, whose control block is then copied to the others. The clock is read by rank
+// 0 while the workers run (1000 x 2000, FP64, 4000 trials with their checks: 4.9 us
+// a trial with a time limit as without, 4.7 with a fixed step; 6.9 and 6.5 when
+// all of those went through rank 0).
 //
 // Where the vectors live (FusedMode, chosen by Engine::choose_fused):
 //   copies  every CTA holds the whole trial x and the whole y of both
@@ -91,6 +94,7 @@ struct alignas(16) FusedCtl {
     int active, parity, pending;
     int accepted;   // the trial before was accepted: its dual is the current one
     int slow;       // the decision goes through rank 0 (see FusedState)
+    int expired;    // the time limit has passed; set by rank 0, never taken back
 };
 
 // The next trial's snapshot of an instance's control block.
@@ -102,7 +106,7 @@ __device__ __forceinline__ void fused_snapshot(const InstanceCtl& c, FusedCtl& f
     f.mult_dual = c.trial_eta * c.trial_omega;
     f.frac = c.avg_frac;
     f.accepted = 0;
-    f.slow = 0;
+    f.slow = 0;     // (expired is the clock's alone)
 }
 
 template <class T, int V>
@@ -223,6 +227,9 @@ __device__ __forceinline__ uint32_t rank_addr(const void* local, uint32_t r) {
 __device__ __forceinline__ void st_cluster(uint32_t addr, double v) {
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
+__device__ __forceinline__ void st_cluster(uint32_t addr, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
@@ -246,21 +253,24 @@ __device__ __forceinline__ int fused_factors(const DeviceOptions& o, int64_t fir
 // the same values): the cases of trial_control that stay inside a check
 // interval. `decide` returns false, with nothing changed, for the rest.
 // ---------------------------------------------------------------------------
+template <bool kLimits>
 struct FusedState {
     double eta, omega_eval, omega_trial, eta_max;   // of the phase's controller
+    double held;          // the trials' step while polishing with a fixed step (else eta is)
     double avg_weight, avg_frac;
     double sums[3];
     int64_t index0;       // iteration index at load
     int64_t to_check;     // accepted trials until the check boundary or the limit
     int parity, pending, rejected;
     int accepted, trials; // since the load
-    bool polish, plain;   // plain: decide may be used at all
+    bool polish;
 
     __device__ __forceinline__ void load(const InstanceCtl& c, const DeviceOptions& o) {
         polish = c.phase == kPhasePolish;
         eta = polish ? c.ctl_eta : c.eta;
         omega_eval = polish ? c.ctl_omega : c.omega;
         omega_trial = polish ? c.trial_omega : c.omega;
+        if (kLimits) held = c.trial_eta;
         eta_max = c.eta_max;
         avg_weight = c.avg_weight;
         avg_frac = c.avg_frac;
@@ -273,7 +283,6 @@ struct FusedState {
         pending = c.pending_avg;
         rejected = c.trials_this_iter;
         accepted = trials = 0;
-        plain = o.adaptive && (polish || !(o.time_limit > 0.0));
     }
 
     // trial_control's changes of `trials` trials.
@@ -282,7 +291,7 @@ struct FusedState {
         c.dbg[0] = sums[0];
         c.dbg[1] = sums[1];
         c.dbg[2] = sums[2];
-        c.trial_eta = eta;
+        c.trial_eta = step(o);
         if (polish) {
             c.ctl_eta = eta;
             c.polish_trials += trials;
@@ -303,6 +312,11 @@ struct FusedState {
         c.trials_this_iter = rejected;
     }
 
+    // The trials' step.
+    __device__ __forceinline__ double step(const DeviceOptions& o) const {
+        return kLimits && polish && !o.adaptive ? held : eta;
+    }
+
     // Iteration index of the trial under way.
     __device__ __forceinline__ int64_t iteration() const { return index0 + accepted; }
 
@@ -310,10 +324,10 @@ struct FusedState {
     __device__ __forceinline__ bool decide(const DeviceOptions& o, const double (&s)[3], const double* factors,
                                            int64_t first, int nfactors) {
         const int64_t k = iteration() - first;
-        if (!plain || k >= nfactors || !(isfinite(s[0]) && isfinite(s[1]) && isfinite(s[2]))) return false;
+        if (k >= nfactors || !(isfinite(s[0]) && isfinite(s[1]) && isfinite(s[2]))) return false;
         double next = eta;
         const bool accept =
-            evaluate_step(next, omega_eval, eta_max, o, s[0], s[1], s[2], iteration(), factors + 2 * k);
+            (kLimits && !o.adaptive) || evaluate_step(next, omega_eval, eta_max, o, s[0], s[1], s[2], iteration(), factors + 2 * k);
         if (accept ? to_check <= 1 : rejected + 1 >= o.max_trials) return false;
         eta = next;
         ++trials;
@@ -328,9 +342,10 @@ struct FusedState {
         rejected = 0;
         ++accepted;
         --to_check;
-        if (o.averaging && eta > 0.0) {   // average_add
-            const double total = avg_weight + eta;
-            avg_frac = eta / total;
+        const double weight = step(o);
+        if (o.averaging && weight > 0.0) {   // average_add
+            const double total = avg_weight + weight;
+            avg_frac = weight / total;
             avg_weight = total;
             pending = 1;
         }
@@ -513,7 +528,10 @@ __device__ __forceinline__ FusedRange fused_setup(const Global& g, const DeviceO
     r.ds1 = g.a.ctas[inf.a_cta_end - 1].slice_end;
     r.ne_p = inf.at_cta_end - inf.at_cta_begin;
     r.ne_d = inf.a_cta_end - inf.a_cta_begin;
-    if (threadIdx.x == 0) sc.so = o;
+    if (threadIdx.x == 0) {
+        sc.so = o;
+        sc.f.expired = 0;
+    }
     if (threadIdx.x < sizeof(InstanceCtl) / 16)
         reinterpret_cast<int4*>(&sc.ctl)[threadIdx.x] = reinterpret_cast<const int4*>(cp)[threadIdx.x];
     for (int e = threadIdx.x; e < r.ne_p; e += kFusedThreads) {
@@ -527,7 +545,10 @@ __device__ __forceinline__ FusedRange fused_setup(const Global& g, const DeviceO
     return r;
 }
 
-// The deciding warp of a CTA, from the first trial to the launch's end.
+// The deciding warp of a CTA, from the first trial to the launch's end. kLimits:
+// there is a time limit or the step is fixed. (Kernels of their own: the few
+// instructions it takes would cost every trial 1 to 4%.)
+template <bool kLimits>
 __device__ __forceinline__ void fused_decider(InstanceCtl* cp, int32_t n_cols, bool fp64, int max_trials,
                                               FusedCta& sc, const FusedSums& sums, const FusedRange& range,
                                               uint32_t C, uint32_t rank) {
@@ -537,8 +558,9 @@ __device__ __forceinline__ void fused_decider(InstanceCtl* cp, int32_t n_cols, b
     InstanceCtl& sctl = sc.ctl;
     // Its registers are never the workers'; its barriers match theirs one for
     // one.
-    FusedState state;
+    FusedState<kLimits> state;
     state.load(sctl, so);
+    const bool timed = kLimits && so.time_limit > 0.0 && sctl.deadline_ns > 0;
     int64_t fac0 = 0;   // the factors kept are of iteration indices fac0, fac0 + 1, ..., nfac of them
     int nfac = 0;
     int widest = 16;   // the butterfly's first step that meets an entry
@@ -552,7 +574,16 @@ __device__ __forceinline__ void fused_decider(InstanceCtl* cp, int32_t n_cols, b
             for (int q = lane; q < 2 * nfac; q += 32) sc.fac[q] = so.step_pow[2 * fac0 + q];
             __syncwarp();
         }
+        // The clock, once a trial, by one lane of one CTA, for all: `expired` is
+        // stored before the first barrier and read between the two, so every CTA
+        // sees the same (after the second, rank 0 may be in the next trial).
+        if (timed && rank == 0 && !state.polish) {
+            const bool over = __shfl_sync(kFull, now_ns() >= sctl.deadline_ns ? 1 : 0, 0) != 0;
+            if (over && static_cast<uint32_t>(lane) < C)
+                st_cluster(rank_addr(&f.expired, static_cast<uint32_t>(lane)), 1);
+        }
         trial_sync(C);
+        const bool expired = timed && f.expired != 0;
         trial_sync(C);
         const double* const sums_p = sums.p[t & 1];
         // k_dual's fixed-order sums (warp_range_sum_deep: a lane's entries in
@@ -571,10 +602,11 @@ __device__ __forceinline__ void fused_decider(InstanceCtl* cp, int32_t n_cols, b
 #pragma unroll
         for (int q = 0; q < 3; ++q) s[q] = __shfl_sync(kFull, s[q], 0);
         const int before = state.accepted;
-        if (state.decide(so, s, sc.fac, fac0, nfac)) {
+        if (!expired && state.decide(so, s, sc.fac, fac0, nfac)) {
             if (lane == 0) {
-                f.mult_primal = state.eta / state.omega_trial;
-                f.mult_dual = state.eta * state.omega_trial;
+                const double step = state.step(so);
+                f.mult_primal = step / state.omega_trial;
+                f.mult_dual = step * state.omega_trial;
                 f.frac = state.avg_frac;
                 f.parity = state.parity;
                 f.pending = state.pending;
@@ -618,7 +650,7 @@ __device__ __forceinline__ void fused_decider(InstanceCtl* cp, int32_t n_cols, b
     }
 }
 
-template <class T, int M, int NL>
+template <class T, int M, int NL, bool kLimits>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w, DeviceOptions o, int vlog,
                                                            int max_trials, FusedShape fs) {
     constexpr bool kCopyX = M == kFusedCopies;
@@ -707,7 +739,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w,
     // Remote shared memory is written only once every CTA of the cluster runs.
     cluster_sync_all();
     if (decider) {
-        fused_decider(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
+        fused_decider<kLimits>(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
         return;
     }
 
@@ -885,7 +917,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused_global(Global g, Wor
     if (decider && lane == 0) fused_snapshot(sc.ctl, f, kFp64);
     cluster_sync_all();
     if (decider) {
-        fused_decider(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
+        fused_decider<true>(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
         return;
     }
     auto publish = [&](double* at, double v) {

@@ -1949,12 +1949,12 @@ namespace {
 // The fused kernel of a shape: staged ones by layout and by whether a worker
 // has one slice a side (the code of one slice is a quarter as long, and a
 // trial is as fast as its instructions come in) or up to kFusedLocal.
-template <class T, int NL>
+template <class T, int NL, bool kLimits>
 auto fused_kernel(int mode) {
     switch (mode) {
-        case kFusedCopies: return k_fused<T, kFusedCopies, NL>;
-        case kFusedHalf: return k_fused<T, kFusedHalf, NL>;
-        default: return k_fused<T, kFusedStaged, NL>;
+        case kFusedCopies: return k_fused<T, kFusedCopies, NL, kLimits>;
+        case kFusedHalf: return k_fused<T, kFusedHalf, NL, kLimits>;
+        default: return k_fused<T, kFusedStaged, NL, kLimits>;
     }
 }
 
@@ -1962,8 +1962,9 @@ template <class T>
 auto fused_kernel(int vw, int cluster, const FusedShape& f) {
     if (f.mode == kFusedGlobal)
         return vw == 4 ? k_fused_global<T, 4> : vw == 2 ? k_fused_global<T, 2> : k_fused_global<T, 1>;
-    return std::max(f.slices_p, f.slices_d) <= cluster * kFusedCtaWorkers ? fused_kernel<T, 1>(f.mode)
-                                                                          : fused_kernel<T, kFusedLocal>(f.mode);
+    const bool one = std::max(f.slices_p, f.slices_d) <= cluster * kFusedCtaWorkers;
+    if (f.limits) return one ? fused_kernel<T, 1, true>(f.mode) : fused_kernel<T, kFusedLocal, true>(f.mode);
+    return one ? fused_kernel<T, 1, false>(f.mode) : fused_kernel<T, kFusedLocal, false>(f.mode);
 }
 
 // The launch configuration of `count` clusters; false where the device

@@ -125,6 +125,7 @@ struct FusedShape {
     int32_t stage_bytes;            // most bytes of a CTA's staged slices
     int32_t copied;                 // most elements of an instance's copied vectors
     int32_t elem;                   // bytes of the launch's working precision
+    int32_t limits;                 // there is a time limit or the step is fixed
 };
 // Dynamic shared memory of a fused CTA: two sets of a warp sum per primal
 // slice, two sums per dual slice, one word per CTA-map entry; then the copied
