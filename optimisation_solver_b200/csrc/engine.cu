@@ -912,10 +912,24 @@ int Engine::timed_position(int k, int slots) const {
 }
 
 // Small instances run the trials of a check interval in one cluster launch
-// per precision (k_fused) instead of two launches per trial slot: up to 16
+// per precision (k_fused) instead of three launches per trial slot: up to 16
 // instances whose slices' warp sums fit a CTA's shared memory, when the
-// device can hold such a cluster. The layout of the vectors (FusedMode) is the
-// first that fits the shared memory of the launch's working precision.
+// device can hold such a cluster. The layout of the vectors is the first
+// that fits the shared memory of the launch's working precision, in the order
+// of the times measured (us a trial with its share of the checks):
+//   up to 8 CTAs   copies (1000 x 2000, 4 CTAs, FP64 5.2, staged 6.0; 2000 x 4000,
+//                  8 CTAs, FP32 5.6, 6.2)
+//   16 CTAs        staged (2000-node flow FP64 9.3, copies 11.4; FP32 8.7, 11.8;
+//                  3000 x 6000, 5 a column, FP64 6.6, 8.4), unless the lines are
+//                  long, with more gathers for each value stored: FP32 from 5
+//                  entries a line on (4000 x 8000, 9 a column: copies 11.4, staged
+//                  12.2; 5 a column 8.1, 7.6), FP64 from 12 (1000 x 2000, 30 a
+//                  column: 10.0, 10.3; 15: 6.8, 6.4)
+// Where nothing can be staged and the lines are short, the two-kernel path is the
+// faster one, but for a few instances of a moderate size at a time (fused and
+// two-kernel: one 8000 x 16000 LP FP64 16.1, 13.5, 100000 x 200000 189, 31; four of
+// 8000 x 16000 19.6, 21.4, of 16000 x 32000 29.5, 25.1; nine of 8000 x 16000, in two waves,
+// 34.8, 26.9). Long lines (V > 1) stay: 3000 x 6000, 30 a column, 25.9, 32.6.
 void Engine::choose_fused() {
     fused_cluster_ = 0;
     fused_shape32_ = fused_shape64_ = FusedShape{};
@@ -932,16 +946,20 @@ void Engine::choose_fused() {
     FusedShape sh{};
     sh.elem = static_cast<int32_t>(sizeof(double));
     sh.limits = dopt_.time_limit > 0.0 || !dopt_.adaptive;
-    int32_t rows = 0, cols_rows = 0;   // most 2 m and 2 m + n of an instance
+    int32_t cols_rows = 0;                        // most 2 m + n of an instance
+    int64_t lines = 0, entries = 0, largest = 0;  // of all; most entries of an instance
     for (int b = 0; b < count_; ++b) {
         const InstanceInfo& inf = info_[static_cast<size_t>(b)];
         sh.slices_p = std::max(sh.slices_p, last(at_ctas_, inf.at_cta_end) - first(at_ctas_, inf.at_cta_begin));
         sh.slices_d = std::max(sh.slices_d, last(a_ctas_, inf.a_cta_end) - first(a_ctas_, inf.a_cta_begin));
         sh.entries_p = std::max(sh.entries_p, inf.at_cta_end - inf.at_cta_begin);
         sh.entries_d = std::max(sh.entries_d, inf.a_cta_end - inf.a_cta_begin);
-        rows = std::max<int32_t>(rows, static_cast<int32_t>(std::min<int64_t>(2 * int64_t(inf.m), INT32_MAX)));
         cols_rows = std::max<int32_t>(
             cols_rows, static_cast<int32_t>(std::min<int64_t>(2 * int64_t(inf.m) + inf.n, INT32_MAX)));
+        const int64_t own = layouts_[spec_.shared_matrix ? 0 : b].a.entries;
+        lines += int64_t(inf.m) + inf.n;
+        entries += own;
+        largest = std::max(largest, own);
     }
     if (fused_smem_bytes(sh) > kFusedMaxSmemHost) return;
     const int V = tuning_.vector_width;
@@ -993,11 +1011,12 @@ void Engine::choose_fused() {
         out.elem = elem;
         if (kFusedLocal * cluster * kFusedCtaWorkers < std::max(sh.slices_p, sh.slices_d)) return out;
         if (!narrow) return out;
-        for (const int mode : {kFusedCopies, kFusedHalf, kFusedStaged}) {
+        const bool copies_first = cluster <= 8 || entries >= (elem == 4 ? 5 : 12) * lines;
+        for (const int mode : {copies_first ? kFusedCopies : kFusedStaged, kFusedStaged}) {
             FusedShape f = out;
             f.mode = mode;
             f.stage_bytes = stage_bytes(mode, elem);
-            f.copied = mode == kFusedCopies ? cols_rows : mode == kFusedHalf ? rows : 0;
+            f.copied = mode == kFusedCopies ? cols_rows : 0;
             if (fused_smem_bytes(f) <= kFusedMaxSmemHost && fits(f)) return f;
         }
         return out;
@@ -1007,6 +1026,11 @@ void Engine::choose_fused() {
     if (mixed_)
         fused_shape32_ = best(static_cast<int>(sizeof(float)),
                               [&](const FusedShape& f) { return fused_max_clusters<float>(V, cluster, f) > 0; });
+    const FusedShape& working = mixed_ ? fused_shape32_ : fused_shape64_;
+    if (working.mode == kFusedGlobal && V == 1 &&
+        !(count_ >= 3 && largest <= std::min<int64_t>(28000 * int64_t(count_), 110000) &&
+          resident(cluster, working) >= count_))
+        return;
     fused_cluster_ = cluster;
 }
 

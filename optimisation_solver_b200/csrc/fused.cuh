@@ -22,23 +22,24 @@
 // a trial with a time limit as without, 4.7 with a fixed step; 6.9 and 6.5 when
 // all of those went through rank 0).
 //
-// Where the vectors live (FusedMode, chosen by Engine::choose_fused):
+// Where the vectors live (chosen by Engine::choose_fused):
 //   copies  every CTA holds the whole trial x and the whole y of both
 //           parities; gathers are local, and the owner lane of a line writes
 //           its new value into all C copies (a slice's lanes own consecutive
 //           lines, so each remote store is one contiguous run). The slices,
 //           the lines' constants, iterates and averages are staged in the
 //           owner's shared memory. No trial touches global memory.
-//   half    as copies, but x is too long: the trial x goes through global
-//           memory (L2), y stays in copies.
-//   staged  both x and y go through L2.
+//   staged  as copies, but x and y go through L2: a gather is slower, a new
+//           value is stored once instead of into every CTA. The better one
+//           for sixteen CTAs and short lines, where a trial has as many stores as
+//           gathers.
 //   global  nothing is staged (more slices than four per warp, or no room).
 // Vectors another CTA writes inside the launch are read through L2 (ld.cg);
 // the barrier's release and acquire order them.
 //
 // Bound by latency: two cluster barriers and three dependent phases a trial.
 // 100 trials, FP64, of a 40 x 70 planted LP (one CTA) 224 us, 1000 x 2000
-// (4 CTAs) 409, a 2000-node flow LP (16 CTAs, half) 863. With three barriers a
+// (4 CTAs) 399, a 2000-node flow LP (16 CTAs, staged) 801. With three barriers a
 // trial, the decision by the workers and 32-bit indices from step-major global
 // slices they were 383, 570 and 1133. Of 1000 x 2000's 7800 cycles a trial
 // the sums and the decision take 2900, the dual gathers 1900, the primal 1100
@@ -653,8 +654,7 @@ __device__ __forceinline__ void fused_decider(InstanceCtl* cp, int32_t n_cols, b
 template <class T, int M, int NL, bool kLimits>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w, DeviceOptions o, int vlog,
                                                            int max_trials, FusedShape fs) {
-    constexpr bool kCopyX = M == kFusedCopies;
-    constexpr bool kCopyY = M == kFusedCopies || M == kFusedHalf;
+    constexpr bool kCopies = M == kFusedCopies;
     constexpr bool kFp64 = sizeof(T) == 8;
     __shared__ alignas(16) FusedCta sc;
     extern __shared__ __align__(16) unsigned char fused_smem[];
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w,
     // Copies: y of both parities, then the trial x.
     T* const yc[2] = {copies, copies + inf.m};
     T* const xc = copies + 2 * inf.m;
-    if (kCopyY)
+    if (kCopies)
         for (int q = threadIdx.x; q < inf.m; q += kFusedThreads) {
             yc[0][q] = yg[0][q];
             yc[1][q] = yg[1][q];
@@ -744,8 +744,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w,
     }
 
     auto primal_sum = [&](const FusedSlice<T>& L, int parity) {
-        const T* y = kCopyY ? yc[parity] : yg[parity];
-        if constexpr (kCopyY) return staged_sum(L, lane, [&](int i) { return y[i]; });
+        const T* y = kCopies ? yc[parity] : yg[parity];
+        if constexpr (kCopies) return staged_sum(L, lane, [&](int i) { return y[i]; });
         else return staged_sum(L, lane, [&](int i) { return __ldcg(y + i); });
     };
     // A slice's warp sums, into every CTA's arrays.
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w,
                 const T gradient = cj + sum;
                 const T upd = smax(loj, smin(prev - mult * tj * gradient, hij));
                 own[32 * (1 + (p ^ 1))] = upd;
-                if (kCopyX) store_copies<T>(xc + j, upd, C);
+                if (kCopies) store_copies<T>(xc + j, upd, C);
                 else xg[p ^ 1][j] = upd;
                 const double d = static_cast<double>(upd - prev);
                 vp[i] = d * d * static_cast<double>(itj);
@@ -795,23 +795,23 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w,
             vd[i][0] = vd[i][1] = 0.0;
             if (i >= nd) continue;
             const FusedSlice<T> L = fused_slice<T>(stage, pd[i]);
-            const T* xt = kCopyX ? xc : xg[p ^ 1];
+            const T* xt = kCopies ? xc : xg[p ^ 1];
             T sum;
-            if constexpr (kCopyX) sum = staged_sum(L, lane, [&](int jj) { return xt[jj]; });
+            if constexpr (kCopies) sum = staged_sum(L, lane, [&](int jj) { return xt[jj]; });
             else sum = staged_sum(L, lane, [&](int jj) { return __ldcg(xt + jj); });
             const int r = L.line(lane);
             if (r >= 0) {
                 T* const own = L.k + 32 * kFusedDualConsts + lane;   // Ax, Ax, average (, y, y)
                 const T sgi = L.k[lane], isi = L.k[32 + lane], loi = L.k[64 + lane], hii = L.k[96 + lane];
                 const T axi = own[32 * p];
-                const T prev = kCopyY ? yc[p][r] : own[32 * (3 + p)];
+                const T prev = kCopies ? yc[p][r] : own[32 * (3 + p)];
                 const T next = sum;
                 const T dact = next - axi;
                 const T ext = next + dact;
                 const T step = smax(dm * sgi, min_dual_step<T>());
                 const T u = prev + step * ext;
                 const T upd = smax(u - step * hii, T(0)) + smin(u - step * loi, T(0));
-                if (kCopyY) {
+                if (kCopies) {
                     store_copies<T>(yc[p ^ 1] + r, upd, C);
                 } else {
                     own[32 * (3 + (p ^ 1))] = upd;
@@ -890,13 +890,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused(Global g, Work<T> w,
         w.AX[0][inf.row_off + r] = own[0];
         w.AX[1][inf.row_off + r] = own[32];
         w.avg_y[inf.row_off + r] = own[64];
-        yg[0][r] = kCopyY ? yc[0][r] : own[96];
-        yg[1][r] = kCopyY ? yc[1][r] : own[128];
+        yg[0][r] = kCopies ? yc[0][r] : own[96];
+        yg[1][r] = kCopies ? yc[1][r] : own[128];
     }
 }
 
 // The same with nothing staged: slices and vectors through L2 in every trial.
-template <class T, int V>
+template <class T, int V, bool kLimits>
 __global__ void __launch_bounds__(kFusedThreads, 1) k_fused_global(Global g, Work<T> w, DeviceOptions o, int,
                                                                   int max_trials, FusedShape fs) {
     constexpr bool kFp64 = sizeof(T) == 8;
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_fused_global(Global g, Wor
     if (decider && lane == 0) fused_snapshot(sc.ctl, f, kFp64);
     cluster_sync_all();
     if (decider) {
-        fused_decider<true>(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
+        fused_decider<kLimits>(cp, inf.n, kFp64, max_trials, sc, sums, range, C, rank);
         return;
     }
     auto publish = [&](double* at, double v) {

@@ -1949,22 +1949,20 @@ namespace {
 // The fused kernel of a shape: staged ones by layout and by whether a worker
 // has one slice a side (the code of one slice is a quarter as long, and a
 // trial is as fast as its instructions come in) or up to kFusedLocal.
-template <class T, int NL, bool kLimits>
-auto fused_kernel(int mode) {
-    switch (mode) {
-        case kFusedCopies: return k_fused<T, kFusedCopies, NL, kLimits>;
-        case kFusedHalf: return k_fused<T, kFusedHalf, NL, kLimits>;
-        default: return k_fused<T, kFusedStaged, NL, kLimits>;
-    }
+template <class T, bool kLimits>
+auto fused_kernel(int vw, int cluster, const FusedShape& f) {
+    if (f.mode == kFusedGlobal)
+        return vw == 4 ? k_fused_global<T, 4, kLimits> : vw == 2 ? k_fused_global<T, 2, kLimits>
+                                                                 : k_fused_global<T, 1, kLimits>;
+    if (std::max(f.slices_p, f.slices_d) <= cluster * kFusedCtaWorkers)
+        return f.mode == kFusedCopies ? k_fused<T, kFusedCopies, 1, kLimits> : k_fused<T, kFusedStaged, 1, kLimits>;
+    return f.mode == kFusedCopies ? k_fused<T, kFusedCopies, kFusedLocal, kLimits>
+                                  : k_fused<T, kFusedStaged, kFusedLocal, kLimits>;
 }
 
 template <class T>
 auto fused_kernel(int vw, int cluster, const FusedShape& f) {
-    if (f.mode == kFusedGlobal)
-        return vw == 4 ? k_fused_global<T, 4> : vw == 2 ? k_fused_global<T, 2> : k_fused_global<T, 1>;
-    const bool one = std::max(f.slices_p, f.slices_d) <= cluster * kFusedCtaWorkers;
-    if (f.limits) return one ? fused_kernel<T, 1, true>(f.mode) : fused_kernel<T, kFusedLocal, true>(f.mode);
-    return one ? fused_kernel<T, 1, false>(f.mode) : fused_kernel<T, kFusedLocal, false>(f.mode);
+    return f.limits ? fused_kernel<T, true>(vw, cluster, f) : fused_kernel<T, false>(vw, cluster, f);
 }
 
 // The launch configuration of `count` clusters; false where the device

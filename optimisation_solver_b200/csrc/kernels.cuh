@@ -116,7 +116,7 @@ template <class T>
 void launch_dual(const Global& g, const Work<T>& w, const DeviceOptions& o, int vw,
                  cudaStream_t s, bool chained = false);
 // Where a fused launch keeps its vectors (fused.cuh).
-enum : int32_t { kFusedGlobal = 0, kFusedStaged = 1, kFusedHalf = 2, kFusedCopies = 3 };
+enum : int32_t { kFusedGlobal = 0, kFusedStaged = 1, kFusedCopies = 2 };
 // The shape of a fused launch's shared memory, over its instances.
 struct FusedShape {
     int32_t mode;                   // kFused*
