@@ -1191,7 +1191,6 @@ last_layer(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 constexpr int kPairStages = 6;
 constexpr int kPairThreads = 256;
 constexpr int kPairSmem = kPairStages * 2 * (BM * BK * 2) + 4 * 32 * 33 * 4 + 1024 + 256;
-constexpr uint32_t kPeerBit = 0xFEFFFFFFu;   // a barrier's shared::cluster address in the even CTA
 
 struct PairArgs {
     int M, N, K;
@@ -1214,12 +1213,13 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
     return r;
 }
 
+// `bar` in the shared::cluster window: of either CTA.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int32_t x,
                                                  int32_t y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar & kPeerBit), "r"(x), "r"(y)
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
         : "memory");
 }
 __device__ __forceinline__ void mma_bf16_pair(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
@@ -1311,8 +1311,9 @@ gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUt
                 if (elect_one()) {
                     // Both CTAs' bytes count on the even CTA's barrier.
                     if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), 4 * kBytes);
-                    tma_load_2d_pair(smem_u32(sa + s * kBytes), &map_a, smem_u32(&full[s]), kb * BK, m0);
-                    tma_load_2d_pair(smem_u32(sb + s * kBytes), &map_b, smem_u32(&full[s]), kb * BK, n0);
+                    const uint32_t fb = map_rank(smem_u32(&full[s]), 0);
+                    tma_load_2d_pair(smem_u32(sa + s * kBytes), &map_a, fb, kb * BK, m0);
+                    tma_load_2d_pair(smem_u32(sb + s * kBytes), &map_b, fb, kb * BK, n0);
                 }
             }
         }
