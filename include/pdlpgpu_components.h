@@ -51,8 +51,8 @@ int32_t pdlpgpu_trial(const pdlpgpu_lp* lp, int32_t precision, const double* tau
  * indices, FP64 values), the vectors of pdlpgpu_trial, the outputs, and
  * `reductions` (3 doubles: sum dx^2/tau, sum dy^2/sigma, dy'A dx). `stream`
  * is a cudaStream_t (NULL = default stream); the call only enqueues work.
- * Scratch is a fixed 192 KiB static device array inside the library, so rows
- * and columns are limited to 8,388,608 each (larger sizes are rejected with an
+ * Scratch is a fixed 56 KiB static device array inside the library. Rows and
+ * columns are limited to 8,388,608 each (larger sizes are rejected with an
  * error), and a NULL pointer that a launch would read or write is rejected
  * before anything is enqueued. The first call in each CUDA context (the
  * device's primary context, again after cudaDeviceReset, or a caller's own

@@ -30,17 +30,15 @@ extern "C" void pdlpgpu_internal_set_error(const char* message);
 namespace {
 
 constexpr int kNaThreads = 256;
-constexpr int kNaMaxCtas = 8192;                    // per half
-constexpr int64_t kNaMaxLines = int64_t(1024) * kNaMaxCtas;   // 8,388,608
+constexpr int64_t kNaMaxLines = 8388608;            // the interface's bound; nothing here depends on it
 constexpr int kNaGridCtas = 148 * 16;               // CTAs of a half at most (each loops over its blocks)
 constexpr int kNaUnroll = 6;                        // entries a thread has in flight
 constexpr int kNaChunk = 2 * kNaUnroll * kNaThreads;   // products in shared memory: 24 KiB
 constexpr int kNaLong = 32;                         // longer pieces of a line are summed by a whole warp
-static_assert(kNaGridCtas <= kNaMaxCtas, "one partial slot per CTA");
 constexpr unsigned kFull = 0xffffffffu;
 
-// Slots [0, kNaMaxCtas): primal partials; then two per dual CTA.
-static __device__ __align__(256) double g_noalloc_scratch[3 * kNaMaxCtas];
+// Slots [0, kNaGridCtas): primal partials; then two per dual CTA.
+static __device__ __align__(256) double g_noalloc_scratch[3 * kNaGridCtas];
 
 // Address of the array in each CUDA context it was looked up in. The key is
 // the context's unique ID, not the device ordinal: after cudaDeviceReset, or
@@ -234,7 +232,7 @@ na_dual(int32_t rows, int per, const int64_t* a_start, const int32_t* a_index, c
             inter += d * dact;
         }
     }
-    double* base = scratch + kNaMaxCtas + 2 * blockIdx.x;
+    double* base = scratch + kNaGridCtas + 2 * blockIdx.x;
     cta_sum(moved, inter, base, base + 1);
 }
 
@@ -246,8 +244,8 @@ na_reduce(int primal_ctas, int dual_ctas, const double* scratch, double* out) {
     double p = 0.0, d = 0.0, it = 0.0;
     for (int k = threadIdx.x; k < primal_ctas; k += kNaThreads) p += scratch[k];
     for (int k = threadIdx.x; k < dual_ctas; k += kNaThreads) {
-        d += scratch[kNaMaxCtas + 2 * k];
-        it += scratch[kNaMaxCtas + 2 * k + 1];
+        d += scratch[kNaGridCtas + 2 * k];
+        it += scratch[kNaGridCtas + 2 * k + 1];
     }
     cta_sum(p, d, out, out + 1);
     __syncthreads();
@@ -348,8 +346,7 @@ extern "C" int32_t pdlpgpu_trial_noalloc(
     double* reductions, void* stream) {
     if (rows < 0 || cols < 0) return fail("pdlpgpu_trial_noalloc: negative dimensions");
     if (rows > kNaMaxLines || cols > kNaMaxLines)
-        return fail("pdlpgpu_trial_noalloc: at most 8388608 rows and 8388608 columns "
-                    "(the static scratch holds 8192 partial sums per half)");
+        return fail("pdlpgpu_trial_noalloc: at most 8388608 rows and 8388608 columns");
     if (!(weight > 0.0)) return fail("pdlpgpu_trial_noalloc: weight must be positive");
     // Every pointer a launch would dereference must be given: NULL is refused
     // here, before anything is enqueued, instead of faulting on the device.
