@@ -867,13 +867,6 @@ bool Engine::start() {
 // ---------------------------------------------------------------------------
 // The iteration loop
 // ---------------------------------------------------------------------------
-template <class T>
-void Engine::enqueue_trial(const Work<T>& w) {
-    launch_primal<T>(g_, w, dopt_, tuning_.vector_width, stream_);
-    launch_dual<T>(g_, w, dopt_, tuning_.vector_width, stream_);
-    launches_ += 3;
-}
-
 void Engine::enqueue_check_stage(bool il_sync) {
     const int V = tuning_.vector_width;
     const bool sync = il_sync && il_;

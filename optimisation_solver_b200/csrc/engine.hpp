@@ -84,8 +84,6 @@ public:
                             double* metrics, double* verdicts);
 
 private:
-    template <class T> void enqueue_trial(const Work<T>& w);
-    template <class T> void enqueue_check(const Work<T>& w);
     bool enqueue_chunk(int slots, bool fp64_stage);
     // One chunk: the captured graph with or without the FP64 trial kernels,
     // as the last poll's count of FP64-stage instances asks.

@@ -231,31 +231,22 @@ __device__ __forceinline__ void load_operand(uint32_t dst, const CUtensorMap* ma
 // gives lane `lane` the four values of row 4 q + lane / 8 from column
 // 4 (lane % 8) on, q < 8, so a warp's accesses are 128-byte row pieces.
 // ---------------------------------------------------------------------------
-// C[z][M][N] = acc (+ bias): a K split's partial, or the product itself.
+// C[z][M][N] = acc: a K split's partial, or the product itself.
 struct EpiStore {
     float* C;
     int64_t split_stride;
-    const float* bias;
     __device__ __forceinline__ const float* sums() const { return C; }
     template <class Acc>
-    __device__ __forceinline__ void block(int z, bool complete, int row0, int col0, int M, int N,
-                                          const Acc& acc) const {
+    __device__ __forceinline__ void block(int z, int row0, int col0, int M, int N, const Acc& acc) const {
         const int lane = threadIdx.x & 31;
-        const float* bias = complete ? this->bias : nullptr;   // not on a sum that more splits will join
         float* out = C + z * split_stride;
         const int col = col0 + 4 * (lane & 7);
         const bool wide = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-        float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (bias != nullptr)
-            for (int k = 0; k < 4; ++k)
-                if (col + k < N) b[k] = bias[col + k];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const int row = row0 + 4 * q + (lane >> 3);
             float v[4];
             acc(q, v);
-            if (bias != nullptr)
-                for (int k = 0; k < 4; ++k) v[k] += b[k];
             float* p = out + static_cast<int64_t>(row) * N + col;
             if (wide) {
                 if (row < M && col < N) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
@@ -363,8 +354,8 @@ constexpr int tile_accs() {
     return tile_smem<kBN, kStages>() > 113 * 1024 ? 512 / kBN : 256 / kBN;
 }
 
-// Warp-specialised: lane 0 of warp 0 loads (it refills a stage as soon as the
-// MMAs that read it have completed), lane 0 of warp 1 issues the MMAs, then
+// Warp-specialised: warp 0 loads (it refills a stage as soon as the MMAs that
+// read it have completed), warp 1 issues the MMAs, each by an elected lane, then
 // all eight warps take the accumulator: warp w rows 32 (w % 4).., columns
 // kBN / 2 (w / 4)... With several splits per CTA each has its own
 // accumulator, and the epilogue adds them in split order; beyond
@@ -506,7 +497,7 @@ __device__ __forceinline__ void tile_product(const CUtensorMap& map_a, const CUt
 #pragma unroll
             for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = sum[j];
             __syncwarp();
-            epi.block(z, g1 == a.splits, row0, n0 + c0, a.M, a.N, [&](int q, float (&v)[4]) {
+            epi.block(z, row0, n0 + c0, a.M, a.N, [&](int q, float (&v)[4]) {
                 const float* t = tile + (4 * q + (lane >> 3)) * 33 + 4 * (lane & 7);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) v[k] = t[k];

@@ -260,10 +260,8 @@ template <> __device__ __forceinline__ const float* matrix_values<float>(const S
 
 
 // ---------------------------------------------------------------------------
-// Primal half (pdhg_kernel.cpp:47-104)
-// ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
-// The trial kernels. A CTA takes every gridDim-th entry of the CTA map, as many
+// The trial kernels: the primal half (pdhg_kernel.cpp:47-104), the dual half and
+// the decision. A CTA takes every gridDim-th entry of the CTA map, as many
 // CTAs as the device holds at once. What starts an entry -- a record per warp
 // (WarpHead) and the instance's step (TrialParams) -- is brought into shared
 // memory for up to kTrialTile entries at once, and an entry's first slots and

@@ -449,7 +449,7 @@ bool plain_gemm(const bf16* A, const bf16* B, float* C, int M, int N, int K, int
     const int64_t ctas = tiles * sp.count, waves = (ctas + 2 * sms - 1) / (2 * sms);
     if (sp.count > 1 && scratch != nullptr && ctas <= kScratchTiles && (ctas <= sms || 3 * waves <= sp.count)) {
         const int64_t total = int64_t(M) * N;
-        const EpiStore epi{scratch, total, nullptr};
+        const EpiStore epi{scratch, total};
         if (!(ctas <= sms ? tile_gemm<128, 6, false, false>(A, B, M, N, K, sp, true, epi, err, s, false, msg)
                           : tile_gemm<128, 3, false, false>(A, B, M, N, K, sp, true, epi, err, s, false, msg)))
             return false;
@@ -458,7 +458,7 @@ bool plain_gemm(const bf16* A, const bf16* B, float* C, int M, int N, int K, int
         return launch(wide ? add_splits<4> : add_splits<1>, dim3(static_cast<unsigned>((threads + 127) / 128)), 128, 0, s,
                       true, 1, scratch, sp.count, total, C);
     }
-    const EpiStore epi{C, 0, nullptr};
+    const EpiStore epi{C, 0};
     if (tiles <= sms || sp.count > 1)
         return tile_gemm<128, 6, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
     return tile_gemm<128, 3, false, false>(A, B, M, N, K, sp, false, epi, err, s, false, msg);
@@ -559,7 +559,7 @@ struct pdlpgpu_mlp {
     template <bool kBMn>
     bool hidden_product(const bf16* A, const bf16* B, int K, Splits& sp) {
         sp = effective_splits(K, splits_for(batch, hidden, K));
-        const EpiStore epi{partial, int64_t(batch) * hidden, nullptr};
+        const EpiStore epi{partial, int64_t(batch) * hidden};
         const int64_t ctas = int64_t((batch + BM - 1) / BM) * ((hidden + 127) / 128) * sp.count;
         return ctas <= sms ? product<6, false, kBMn>(A, B, batch, hidden, K, sp, epi)
                            : product<3, false, kBMn>(A, B, batch, hidden, K, sp, epi);
@@ -641,7 +641,7 @@ struct pdlpgpu_mlp {
     // as they lie, into `grad`.
     bool weight_gradient(const bf16* D, const bf16* A, int rows, int cols, float* grad) {
         return grad == nullptr || product<3, true, true>(D, A, rows, cols, batch, effective_splits(batch, 1),
-                                                         EpiStore{grad, 0, nullptr});
+                                                         EpiStore{grad, 0});
     }
     bool adam_layer(AdamLayer& L, const bf16* D, const bf16* A, int rows, int cols, float* p, float* m, float* v,
                     bf16* h) {
