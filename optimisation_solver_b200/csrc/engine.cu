@@ -922,7 +922,9 @@ int Engine::timed_position(int k, int slots) const {
 // faster one, but for a few instances of a moderate size at a time (fused and
 // two-kernel: one 8000 x 16000 LP FP64 16.1, 13.5, 100000 x 200000 189, 31; four of
 // 8000 x 16000 19.6, 21.4, of 16000 x 32000 29.5, 25.1; nine of 8000 x 16000, in two waves,
-// 34.8, 26.9). Long lines (V > 1) stay: 3000 x 6000, 30 a column, 25.9, 32.6.
+// 34.8, 26.9). Long lines (V > 1), of which a worker has fewer, stay up to 400,000
+// entries (30 a column, FP64: 3000 x 6000 24.9, 32.6, 6000 x 12000 46.8, 50.6, 10000 x
+// 20000 76.4, 67.2; FP32 20000 x 40000 137, 42).
 void Engine::choose_fused() {
     fused_cluster_ = 0;
     fused_shape32_ = fused_shape64_ = FusedShape{};
@@ -1020,10 +1022,11 @@ void Engine::choose_fused() {
         fused_shape32_ = best(static_cast<int>(sizeof(float)),
                               [&](const FusedShape& f) { return fused_max_clusters<float>(V, cluster, f) > 0; });
     const FusedShape& working = mixed_ ? fused_shape32_ : fused_shape64_;
-    if (working.mode == kFusedGlobal && V == 1 &&
-        !(count_ >= 3 && largest <= std::min<int64_t>(28000 * int64_t(count_), 110000) &&
-          resident(cluster, working) >= count_))
-        return;
+    if (working.mode == kFusedGlobal) {
+        const bool few = count_ >= 3 && largest <= std::min<int64_t>(28000 * int64_t(count_), 110000) &&
+                         resident(cluster, working) >= count_;
+        if (V == 1 ? !few : largest > 400000) return;
+    }
     fused_cluster_ = cluster;
 }
 

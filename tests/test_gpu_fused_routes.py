@@ -20,7 +20,7 @@ SHAPES = [
     (4090, 8180, 5, 1), (4110, 8220, 5, 1),      # a second slice a worker
     (6500, 13000, 5, 1), (16300, 32700, 5, 1), (17000, 34000, 5, 1),   # nothing staged; more slices than four a worker
     (8000, 16000, 5, 2), (8000, 16000, 5, 3), (10000, 20000, 5, 3), (10000, 20000, 5, 4), (8000, 16000, 5, 9),
-    (30000, 60000, 3, 1), (300, 5000, 40, 1), (1200, 1500, 60, 1),
+    (30000, 60000, 3, 1), (300, 5000, 40, 1), (1200, 1500, 60, 1), (6500, 13000, 30, 1), (7000, 14000, 30, 1),
 ]
 
 
