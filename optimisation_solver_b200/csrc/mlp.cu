@@ -135,40 +135,75 @@ __global__ void to_bf16(const float* src, bf16* dst, int64_t n) {
 }
 
 // --- codec between LP instances and the network -----------------------------
-// One row of the batch per blockIdx.y, blockIdx.x * blockDim.x elements of it
-// at a time, four per thread: no element divides its index, and a thread has
-// four independent loads in flight. HBM-bound (20 bytes an element in, 8 to 12
-// out); the flow family's 256 instances of 22,000 parameters.
+// A CTA takes 1024 elements, four a thread, whose loads are in flight together: of
+// long rows neighbouring elements of one row, so that no element divides its
+// index; of rows of up to 512 elements whatever follows in the batch, with one
+// division a thread. HBM-bound (20 bytes an element in, 8 to 12 out). Features of
+// the flow family's 256 instances of 22,000 parameters: 10.4 us (a division per
+// element 20.8); 65,536 rows of 8: 6.8, of 300 62 (a CTA a row 45 and 76, a
+// division per element 6.8 and 68).
 constexpr int kCodecThreads = 256;
 constexpr int kCodecItems = 4;
-inline dim3 codec_grid(int64_t width, int rows) {
-    const int64_t per = kCodecThreads * kCodecItems;
-    return dim3(static_cast<unsigned>((width + per - 1) / per), static_cast<unsigned>(rows < 65535 ? rows : 65535));
-}
+constexpr int kCodecShort = 512;
+struct CodecLaunch {
+    bool wide;
+    dim3 grid;
+    CodecLaunch(int64_t width, int B) : wide(width > kCodecShort) {
+        const int64_t per = kCodecThreads * kCodecItems, total = wide ? width : width * B;
+        grid = dim3(static_cast<unsigned>((total + per - 1) / per),
+                    wide ? static_cast<unsigned>(B < 65535 ? B : 65535) : 1u);
+    }
+};
 
-// f(b, j) for the CTA's elements j < width of its rows b < B: `load` of all
-// items before `store` of the first.
-template <class Load, class Store>
+// f(b, j) for the CTA's elements j < width of rows b < B: `load` of all items
+// before `store` of the first.
+template <bool kWide, class Load, class Store>
 __device__ __forceinline__ void codec_rows(int B, int width, Load load, Store store) {
-    const int j0 = blockIdx.x * (kCodecThreads * kCodecItems) + threadIdx.x;
-    for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    if constexpr (kWide) {
+        const int j0 = blockIdx.x * (kCodecThreads * kCodecItems) + threadIdx.x;
+        for (int b = blockIdx.y; b < B; b += gridDim.y) {
+            decltype(load(0, 0)) v[kCodecItems];
+#pragma unroll
+            for (int k = 0; k < kCodecItems; ++k)
+                if (j0 + k * kCodecThreads < width) v[k] = load(b, j0 + k * kCodecThreads);
+#pragma unroll
+            for (int k = 0; k < kCodecItems; ++k)
+                if (j0 + k * kCodecThreads < width) store(b, j0 + k * kCodecThreads, v[k]);
+        }
+    } else {
+        const uint64_t t = uint64_t(blockIdx.x) * (kCodecThreads * kCodecItems) + threadIdx.x;
+        const uint64_t b0 = (t >> 32) == 0 ? static_cast<uint32_t>(t) / static_cast<uint32_t>(width) : t / width;
+        const int step_b = kCodecThreads / width, step_j = kCodecThreads % width;
+        int b[kCodecItems], j[kCodecItems];
+        b[0] = static_cast<int>(b0 < static_cast<uint64_t>(B) ? b0 : B);
+        j[0] = static_cast<int>(t - b0 * width);
+#pragma unroll
+        for (int k = 1; k < kCodecItems; ++k) {
+            j[k] = j[k - 1] + step_j;
+            b[k] = b[k - 1] >= B - step_b ? B : b[k - 1] + step_b;
+            if (j[k] >= width) {
+                j[k] -= width;
+                b[k] += b[k] < B ? 1 : 0;
+            }
+        }
         decltype(load(0, 0)) v[kCodecItems];
 #pragma unroll
         for (int k = 0; k < kCodecItems; ++k)
-            if (j0 + k * kCodecThreads < width) v[k] = load(b, j0 + k * kCodecThreads);
+            if (b[k] < B) v[k] = load(b[k], j[k]);
 #pragma unroll
         for (int k = 0; k < kCodecItems; ++k)
-            if (j0 + k * kCodecThreads < width) store(b, j0 + k * kCodecThreads, v[k]);
+            if (b[k] < B) store(b[k], j[k], v[k]);
     }
 }
 
 // Features: standardised instance parameters, BF16, zero-padded to `padded`.
 // The parameters are the P of `first` and the Q of `second`, in that order
 // (one array has Q = 0).
+template <bool kWide>
 __global__ void __launch_bounds__(kCodecThreads)
-encode_features(const double* first, int P, const double* second, int Q, int B, int padded, const float* mean,
+encode_features(int B, int padded, const double* first, int P, const double* second, int Q, const float* mean,
                 const float* inv_std, bf16* out) {
-    codec_rows(
+    codec_rows<kWide>(
         B, padded,
         [&](int b, int k) {
             const int64_t r = b;
@@ -180,26 +215,28 @@ encode_features(const double* first, int P, const double* second, int Q, int B, 
 }
 
 // Targets: primal / scale, standardised dual, standardised log weight, zeros.
+template <bool kWide>
 __global__ void __launch_bounds__(kCodecThreads)
-encode_targets(const double* x, const double* y, const double* w, int B, int n, int m, int O, const double* scale,
+encode_targets(int B, int O, const double* x, const double* y, const double* w, int n, int m, const double* scale,
                const float* ymean, const float* yinv, float wmean, float winv, float* out) {
-    codec_rows(
+    codec_rows<kWide>(
         B, O,
         [&](int b, int j) {
             const int64_t r = b;
             if (j < n) return static_cast<float>(x[r * n + j] / scale[j]);
             if (j < n + m) return (static_cast<float>(y[r * m + (j - n)]) - ymean[j - n]) * yinv[j - n];
-            return j == n + m ? (logf(static_cast<float>(w[b])) - wmean) * winv : 0.0f;
+            return j == n + m ? (logf(static_cast<float>(w[r])) - wmean) * winv : 0.0f;
         },
         [&](int b, int j, float v) { out[static_cast<int64_t>(b) * O + j] = v; });
 }
 
 // Warm start from network outputs: x = clamp(out, 0, 1) * scale, y and the
 // weight de-standardised.
+template <bool kWide>
 __global__ void __launch_bounds__(kCodecThreads)
-decode_warmstart(const float* out, int B, int n, int m, int O, const double* scale, const float* ymean,
+decode_warmstart(int B, const float* out, int n, int m, int O, const double* scale, const float* ymean,
                  const float* ystd, float wmean, float wstd, double* wx, double* wy, double* ww) {
-    codec_rows(
+    codec_rows<kWide>(
         B, n + m + 1,
         [&](int b, int j) {
             const float v = out[static_cast<int64_t>(b) * O + j];
@@ -211,7 +248,7 @@ decode_warmstart(const float* out, int B, int n, int m, int O, const double* sca
             const int64_t r = b;
             if (j < n) wx[r * n + j] = v;
             else if (j < n + m) wy[r * m + (j - n)] = v;
-            else ww[b] = v;
+            else ww[r] = v;
         });
 }
 
@@ -921,8 +958,9 @@ int32_t pdlpgpu_gemm_time(int32_t M, int32_t N, int32_t K, const uint16_t* A, co
 int32_t pdlpgpu_encode_features(const double* params, int32_t batch, int32_t count, int32_t padded,
                                 const float* mean, const float* inv_std, uint16_t* out) {
     if (batch <= 0 || count <= 0 || padded < count) return fail("encode_features: bad sizes");
-    encode_features<<<codec_grid(padded, batch), kCodecThreads>>>(
-        params, count, nullptr, 0, batch, padded, mean, inv_std, reinterpret_cast<bf16*>(out));
+    const CodecLaunch c(padded, batch);
+    (c.wide ? encode_features<true> : encode_features<false>)<<<c.grid, kCodecThreads>>>(
+        batch, padded, params, count, nullptr, 0, mean, inv_std, reinterpret_cast<bf16*>(out));
     return cudaGetLastError() == cudaSuccess ? 0 : fail("encode_features: launch failed");
 }
 
@@ -932,8 +970,9 @@ int32_t pdlpgpu_encode_feature_pair(const double* first, int32_t first_count, co
     const int64_t count = static_cast<int64_t>(first_count) + second_count;
     if (batch <= 0 || first_count <= 0 || second_count <= 0 || padded < count)
         return fail("encode_feature_pair: bad sizes");
-    encode_features<<<codec_grid(padded, batch), kCodecThreads>>>(
-        first, first_count, second, second_count, batch, padded, mean, inv_std, reinterpret_cast<bf16*>(out));
+    const CodecLaunch c(padded, batch);
+    (c.wide ? encode_features<true> : encode_features<false>)<<<c.grid, kCodecThreads>>>(
+        batch, padded, first, first_count, second, second_count, mean, inv_std, reinterpret_cast<bf16*>(out));
     return cudaGetLastError() == cudaSuccess ? 0 : fail("encode_feature_pair: launch failed");
 }
 
@@ -943,9 +982,10 @@ int32_t pdlpgpu_encode_targets(const double* primal, const double* dual, const d
                                const float* dual_inv_std, float weight_mean, float weight_inv_std,
                                float* targets) {
     if (batch <= 0 || out_width < n + m + 1) return fail("encode_targets: bad sizes");
-    encode_targets<<<codec_grid(out_width, batch), kCodecThreads>>>(
-        primal, dual, weight, batch, n, m, out_width, primal_scale, dual_mean, dual_inv_std,
-        weight_mean, weight_inv_std, targets);
+    const CodecLaunch c(out_width, batch);
+    (c.wide ? encode_targets<true> : encode_targets<false>)<<<c.grid, kCodecThreads>>>(
+        batch, out_width, primal, dual, weight, n, m, primal_scale, dual_mean, dual_inv_std, weight_mean,
+        weight_inv_std, targets);
     return cudaGetLastError() == cudaSuccess ? 0 : fail("encode_targets: launch failed");
 }
 
@@ -954,9 +994,10 @@ int32_t pdlpgpu_decode_warmstart(const float* outputs, int32_t batch, int32_t n,
                                  const float* dual_mean, const float* dual_std, float weight_mean,
                                  float weight_std, double* primal, double* dual, double* weight) {
     if (batch <= 0 || out_width < n + m + 1) return fail("decode_warmstart: bad sizes");
-    decode_warmstart<<<codec_grid(static_cast<int64_t>(n) + m + 1, batch), kCodecThreads>>>(
-        outputs, batch, n, m, out_width, primal_scale, dual_mean, dual_std, weight_mean, weight_std,
-        primal, dual, weight);
+    const CodecLaunch c(static_cast<int64_t>(n) + m + 1, batch);
+    (c.wide ? decode_warmstart<true> : decode_warmstart<false>)<<<c.grid, kCodecThreads>>>(
+        batch, outputs, n, m, out_width, primal_scale, dual_mean, dual_std, weight_mean, weight_std, primal, dual,
+        weight);
     return cudaGetLastError() == cudaSuccess ? 0 : fail("decode_warmstart: launch failed");
 }
 
