@@ -1176,8 +1176,8 @@ last_layer(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 // TMEM columns hold two accumulators, so a tile's epilogue (warps 4-7 of both
 // CTAs) runs under the next tile's main loop. Bound by the copies into shared
 // memory, 32 KB an SM and K block (about 80 bytes a cycle), and at 8192^3 by
-// power: 730 us, 1505 TFLOP/s, 0.91 of the measured dense BF16 peak; the
-// 128 x 128 tiles of one CTA took 933 us there.
+// power: 720 to 742 us, 1482 to 1527 TFLOP/s, 0.89 to 0.92 of the measured dense
+// BF16 peak; the 128 x 128 tiles of one CTA took 931 us there.
 // ---------------------------------------------------------------------------
 constexpr int kPairStages = 6;
 constexpr int kPairThreads = 256;

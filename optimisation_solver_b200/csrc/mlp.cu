@@ -592,7 +592,8 @@ struct pdlpgpu_mlp {
 
     // partial[z] of a [batch][hidden] product over K, and its splits. With at
     // most one CTA per SM the ring is six stages deep (the copies in flight
-    // bound a long K): 22,000 inputs, 512 wide, batch 256.
+    // bound a long K): 22,000 inputs, 512 wide, batch 256. More CTAs go two to an
+    // SM with three stages, as in plain_gemm.
     template <bool kBMn>
     bool hidden_product(const bf16* A, const bf16* B, int K, Splits& sp) {
         sp = effective_splits(K, splits_for(batch, hidden, K));
