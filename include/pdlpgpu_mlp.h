@@ -10,7 +10,8 @@
  * then runs from the prediction to the same tolerance; the better of the
  * prediction and the cold start by KKT score is used (pdlpgpu_warmstart).
  *
- * All tensors are device pointers, row-major:
+ * All tensors are device pointers, row-major (outputs and gradients in host
+ * memory that is not pinned are refused):
  *   inputs   [batch][in]   BF16 (uint16 bit patterns)
  *   outputs  [batch][out]  FP32
  *   targets  [batch][out]  FP32, with per-output loss weights [out]

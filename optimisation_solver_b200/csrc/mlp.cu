@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <initializer_list>
 #include <mutex>
 #include <random>
 #include <string>
@@ -756,6 +757,23 @@ struct pdlpgpu_mlp {
         to_bf16<<<grid_for(int64_t(out) * hidden), 256, 0, stream>>>(W3, W3h, int64_t(out) * hidden);
     }
 
+    // Whether the kernels can store to a caller's array (null: not asked for);
+    // host memory that is not mapped for the device is refused here, instead of
+    // faulting there.
+    bool writable(std::initializer_list<const float*> arrays) {
+        for (const float* p : arrays) {
+            if (p == nullptr) continue;
+            cudaPointerAttributes a;
+            if (cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type != cudaMemoryTypeUnregistered &&
+                (reinterpret_cast<uintptr_t>(p) & 3) == 0)
+                continue;
+            cudaGetLastError();
+            msg = "outputs must be float arrays in device memory";
+            return false;
+        }
+        return true;
+    }
+
     // Waits for the call; false on a CUDA error or a pipeline timeout.
     bool finish(const char* what, float* loss) {
         if (cudaMemcpyAsync(report, report_dev, sizeof(Report), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
@@ -848,6 +866,7 @@ int32_t pdlpgpu_mlp_forward(pdlpgpu_mlp* m, const uint16_t* inputs, float* outpu
     if (!m) return -1;
     cudaSetDevice(m->device);
     m->launches = 0;
+    if (outputs == nullptr || !m->writable({outputs})) return fail("mlp forward: outputs must be float arrays in device memory");
     if (!m->wait_for_caller()) return fail("mlp forward: stream wait failed");
     if (!m->forward(reinterpret_cast<const bf16*>(inputs), outputs)) return fail("mlp forward: " + m->msg);
     if (!m->finish("mlp forward", nullptr)) return fail(m->msg);
@@ -860,6 +879,7 @@ int32_t pdlpgpu_mlp_gradients(pdlpgpu_mlp* m, const uint16_t* inputs, const floa
     if (!m) return -1;
     cudaSetDevice(m->device);
     m->launches = 0;
+    if (!m->writable({dW1, db1, dW2, db2, dW3, db3})) return fail("mlp gradients: " + m->msg);
     if (!m->wait_for_caller()) return fail("mlp gradients: stream wait failed");
     const pdlpgpu_mlp::Gradients g{dW1, db1, dW2, db2, dW3, db3};
     if (!m->step_or_gradients(reinterpret_cast<const bf16*>(inputs), targets, w, false, 0.0f, g))

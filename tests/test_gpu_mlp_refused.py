@@ -1,5 +1,7 @@
-"""A training step that is refused leaves the model as it was: the step after
-it is the step of a model that never saw the refused call, bit for bit."""
+"""Calls that are refused on the host. A training step that is refused leaves the
+model as it was: the step after it is the step of a model that never saw the
+refused call, bit for bit. Outputs that the device cannot store to (host memory
+that is not pinned) are an error of the call, and the model goes on working."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -41,3 +43,35 @@ def test_a_refused_step_does_not_count(refused_after):
     assert losses == want_losses
     for k in shapes:
         assert torch.equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("where", ["host", "pinned"])
+def test_outputs_in_host_memory(where):
+    import torch
+    from optimisation_solver_b200.mlp import Mlp
+
+    inputs, hidden, outputs, batch = 64, 64, 128, 8
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(9)
+    x = torch.randn((batch, inputs), generator=gen, device="cuda").to(torch.bfloat16)
+    target = torch.randn((batch, outputs), generator=gen, device="cuda")
+    weight = torch.rand(outputs, generator=gen, device="cuda")
+    net = Mlp(inputs, hidden, outputs, batch, seed=1)
+    want, want_grad = torch.empty((batch, outputs), device="cuda"), torch.empty((hidden, inputs), device="cuda")
+    net.forward(x, want)
+    net.gradients(x, target, weight, {"W1": want_grad})
+    out, grad = torch.zeros((batch, outputs)), torch.zeros((hidden, inputs))
+    if where == "host":
+        with pytest.raises(RuntimeError, match="device memory"):
+            net.forward(x, out)
+        with pytest.raises(RuntimeError, match="device memory"):
+            net.gradients(x, target, weight, {"W1": grad})
+        assert not out.any() and not grad.any()
+        again = torch.empty_like(want)
+        net.forward(x, again)
+        assert torch.equal(again, want)
+    else:
+        out, grad = out.pin_memory(), grad.pin_memory()
+        net.forward(x, out)
+        net.gradients(x, target, weight, {"W1": grad})
+        assert torch.equal(out, want.cpu()) and torch.equal(grad, want_grad.cpu())
